@@ -1349,7 +1349,8 @@ int ribn_argmax(ribn_ctx* ctx, const float* logits_device, uint32_t members, uin
     Failure f = check_device_pointer(ctx, logits_device, "logits");
     if (f.status == RIBN_OK) f = check_device_pointer(ctx, out_device, "output");
     if (f.status != RIBN_OK) return record(ctx, f);
-    const cudaError_t e = ribn::launch_argmax(logits_device, static_cast<int>(members), length, out_device, ctx->stream);
+    const cudaError_t e = ribn::launch_argmax(logits_device, static_cast<int>(members), length, out_device, ctx->tickets, kTicketCount,
+                                              ctx->sm_count, ctx->stream);
     if (e != cudaSuccess) return record_cuda(ctx, e, "argmax launch");
     return RIBN_OK;
 }

@@ -242,7 +242,9 @@ cudaError_t launch_attention_decode(const LayerAttentionArgs& args, void* out, b
 cudaError_t launch_silu_mul(const float* gate, const float* up, void* out, bool out_bf16, uint64_t members, uint64_t length, uint64_t in_stride,
                             int sm_count, cudaStream_t stream);
 cudaError_t launch_residual_add(float* y, const float* x, uint64_t total, int sm_count, cudaStream_t stream);
-cudaError_t launch_argmax(const float* logits, int members, uint64_t length, uint32_t* out, cudaStream_t stream);
+// `counters`: the context's zero-initialised counters (left zero), for rows that several CTAs share.
+cudaError_t launch_argmax(const float* logits, int members, uint64_t length, uint32_t* out, unsigned int* counters, int counter_count, int sm_count,
+                          cudaStream_t stream);
 
 // One CTA polls an mbarrier nobody arrives at, at most `polls` times, then records kDeviceWaitTimeout in *status.
 cudaError_t launch_bounded_wait_selftest(int* status, uint32_t polls, cudaStream_t stream);

@@ -57,76 +57,103 @@ __global__ void __launch_bounds__(256) embedding_kernel(const uint8_t* __restric
 }
 
 // ---------------------------------------------------------------- head norm + rope + cache append
-// grid (q_heads + 2 kv_heads, members), head_dim threads.  Blocks [0, q_heads) rewrite a query head in
-// place; [q_heads, q_heads + kv_heads) normalise and rotate a key head into the f16 cache; the rest
-// convert a value head into the cache.
-__global__ void __launch_bounds__(256) qk_norm_rope_append_kernel(float* __restrict__ q, const float* __restrict__ k,
-                                                                  const float* __restrict__ v, const float* __restrict__ q_norm,
-                                                                  const float* __restrict__ k_norm, float eps,
-                                                                  const int* __restrict__ positions, int q_heads, int kv_heads,
-                                                                  int head_dim, int rot_pairs, float base, __half* __restrict__ k_cache,
-                                                                  __half* __restrict__ v_cache, long long max_context, int shared_cache,
-                                                                  int* __restrict__ status) {
+// grid (ceil((q_heads + 2 kv_heads) / 8), members), a warp per head of 128 values, four per lane.  Heads [0, q_heads) rewrite a
+// query head in place; [q_heads, q_heads + kv_heads) normalise and rotate a key head into the f16 cache; the rest convert a
+// value head into the cache.  The angles depend on the member and the pair only: the CTA works them out once for its eight
+// heads (a power, a sine and a cosine per pair).  A CTA per head, every thread with its own three of them, took 28 us for 512
+// members of 48 heads.
+constexpr int kHeadDim = 128;
+constexpr int kRopeWarps = 8;
+
+__global__ void __launch_bounds__(kRopeWarps * 32) qk_norm_rope_append_kernel(float* __restrict__ q, const float* __restrict__ k,
+                                                                              const float* __restrict__ v, const float* __restrict__ q_norm,
+                                                                              const float* __restrict__ k_norm, float eps,
+                                                                              const int* __restrict__ positions, int q_heads, int kv_heads,
+                                                                              int rot_pairs, float base, __half* __restrict__ k_cache,
+                                                                              __half* __restrict__ v_cache, long long max_context, int shared_cache,
+                                                                              int* __restrict__ status) {
     pdl_launch_dependents();
     pdl_wait_prior();   // inputs come from the kernels before this one in the stream
-    __shared__ float values[256];
-    __shared__ float warp_sums[8];
+    __shared__ float sines[kHeadDim / 2], cosines[kHeadDim / 2];
+    __shared__ float values[kRopeWarps][kHeadDim];
     const int member = blockIdx.y;
-    const int t = threadIdx.x;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int head = blockIdx.x * kRopeWarps + warp;
     const int position = positions[member];
-    int head = blockIdx.x;
-    const float* source;
+    const float* source = nullptr;
     const float* norm = nullptr;
     bool rotate = true;
     __half* cache = nullptr;
     float* in_place = nullptr;
     if (head < q_heads) {
-        in_place = q + (static_cast<size_t>(member) * q_heads + head) * head_dim;
+        in_place = q + (static_cast<size_t>(member) * q_heads + head) * kHeadDim;
         source = in_place;
         norm = q_norm;
     } else if (head < q_heads + kv_heads) {
         head -= q_heads;
-        source = k + (static_cast<size_t>(member) * kv_heads + head) * head_dim;
+        source = k + (static_cast<size_t>(member) * kv_heads + head) * kHeadDim;
         norm = k_norm;
         cache = k_cache;
-    } else {
+    } else if (head < q_heads + 2 * kv_heads) {
         head -= q_heads + kv_heads;
-        source = v + (static_cast<size_t>(member) * kv_heads + head) * head_dim;
+        source = v + (static_cast<size_t>(member) * kv_heads + head) * kHeadDim;
         rotate = false;
         cache = v_cache;
     }
-    float x = source[t];
-    if (norm != nullptr) {
-        float sum = x * x;
+    float x[4] = {0.0f, 0.0f, 0.0f, 0.0f};   // dims lane + 32 j
+    if (source != nullptr) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        if ((t & 31) == 0) warp_sums[t >> 5] = sum;
-        __syncthreads();
+        for (int j = 0; j < 4; ++j) x[j] = source[lane + 32 * j];
+    }
+    if (threadIdx.x < rot_pairs) {
+        const int pair = threadIdx.x;
+        const float theta = static_cast<float>(position) * powf(base, -(2.0f * static_cast<float>(pair)) / (2.0f * static_cast<float>(rot_pairs)));
+        sines[pair] = sinf(theta);
+        cosines[pair] = cosf(theta);
+    }
+    __syncthreads();
+    if (source == nullptr) return;
+    if (norm != nullptr) {
         float total = 0.0f;
-        for (int wi = 0; wi < (head_dim + 31) / 32; ++wi) total += warp_sums[wi];
-        const float inverse = rsqrtf(total / static_cast<float>(head_dim) + eps);
-        x = x * inverse * norm[t];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            float sum = x[j] * x[j];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            total += sum;
+        }
+        const float inverse = rsqrtf(total / static_cast<float>(kHeadDim) + eps);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) x[j] = x[j] * inverse * norm[lane + 32 * j];
     }
     if (rotate && rot_pairs > 0) {
-        values[t] = x;
-        __syncthreads();
-        if (t < 2 * rot_pairs) {
-            const int pair = t < rot_pairs ? t : t - rot_pairs;
-            const float theta = static_cast<float>(position) * powf(base, -(2.0f * static_cast<float>(pair)) / (2.0f * static_cast<float>(rot_pairs)));
-            const float sin_theta = sinf(theta);
-            const float cos_theta = cosf(theta);
-            const float x0 = values[pair];
-            const float x1 = values[pair + rot_pairs];
-            x = t < rot_pairs ? x0 * cos_theta - x1 * sin_theta : x0 * sin_theta + x1 * cos_theta;
+        float* own = values[warp];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) own[lane + 32 * j] = x[j];
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int d = lane + 32 * j;
+            if (d < 2 * rot_pairs) {
+                const int pair = d < rot_pairs ? d : d - rot_pairs;
+                const float sin_theta = sines[pair];
+                const float cos_theta = cosines[pair];
+                const float x0 = own[pair];
+                const float x1 = own[pair + rot_pairs];
+                x[j] = d < rot_pairs ? x0 * cos_theta - x1 * sin_theta : x0 * sin_theta + x1 * cos_theta;
+            }
         }
     }
     if (in_place != nullptr) {
-        in_place[t] = x;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) in_place[lane + 32 * j] = x[j];
     } else if (position >= 0 && position < max_context) {
         // a prefill chunk: the members are consecutive tokens of one sequence and append to the same cache
         const long long sequence = shared_cache ? 0 : member;
-        cache[((sequence * kv_heads + head) * max_context + position) * head_dim + t] = __float2half_rn(x);
-    } else if (t == 0) {
+        __half* slot = cache + ((sequence * kv_heads + head) * max_context + position) * kHeadDim;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) slot[lane + 32 * j] = __float2half_rn(x[j]);
+    } else if (lane == 0) {
         // The position comes from device memory (a replayed graph advances it): outside the cache nothing is
         // stored and the context's status word says so.
         atomicExch(status, kDevicePositionOutOfRange);
@@ -400,83 +427,121 @@ __global__ void __launch_bounds__(kAttnHeadDim) attention_combine_kernel(const f
 
 // ---------------------------------------------------------------- elementwise
 // out[m][i] = silu(gate[m][i]) * up[m][i]; gate and up rows are `in_stride` floats apart (they may be the two
-// halves of one [members][2 * length] GEMV output), out rows are `length` apart.
-template <bool OUT_BF16>
+// halves of one [members][2 * length] GEMV output), out rows are `length` apart.  Grid (pieces of a row, members); four
+// neighbouring values per thread where rows keep 16-byte boundaries (VECTOR), one otherwise.  Bound by memory: 512 rows of
+// 12288 took 22.8 us with one value and one 64-bit division per thread and step.
+template <bool OUT_BF16, bool VECTOR>
 __global__ void __launch_bounds__(256) silu_mul_kernel(const float* __restrict__ gate, const float* __restrict__ up, void* __restrict__ out,
-                                                       unsigned long long length, unsigned long long in_stride, unsigned long long total) {
+                                                       unsigned long long length, unsigned long long in_stride, unsigned int first_member) {
     pdl_launch_dependents();
     pdl_wait_prior();   // inputs come from the kernels before this one in the stream
-    for (unsigned long long i = static_cast<unsigned long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
-         i += static_cast<unsigned long long>(gridDim.x) * blockDim.x) {
-        const unsigned long long member = i / length;
-        const unsigned long long column = i - member * length;
-        const float value = gate[member * in_stride + column];
-        const float product = (value / (1.0f + expf(-value))) * up[member * in_stride + column];
-        if constexpr (OUT_BF16) static_cast<__nv_bfloat16*>(out)[i] = __float2bfloat16_rn(product);
-        else static_cast<float*>(out)[i] = product;
+    constexpr int kWidth = VECTOR ? 4 : 1;
+    const unsigned long long member = static_cast<unsigned long long>(first_member) + blockIdx.y;
+    const float* gate_row = gate + member * in_stride;
+    const float* up_row = up + member * in_stride;
+    for (unsigned long long i = (static_cast<unsigned long long>(blockIdx.x) * blockDim.x + threadIdx.x) * kWidth; i < length;
+         i += static_cast<unsigned long long>(gridDim.x) * blockDim.x * kWidth) {
+        float g[kWidth], u[kWidth], product[kWidth];
+        if constexpr (VECTOR) {
+            const float4 gv = *reinterpret_cast<const float4*>(gate_row + i), uv = *reinterpret_cast<const float4*>(up_row + i);
+            g[0] = gv.x; g[1] = gv.y; g[2] = gv.z; g[3] = gv.w;
+            u[0] = uv.x; u[1] = uv.y; u[2] = uv.z; u[3] = uv.w;
+        } else {
+            g[0] = gate_row[i];
+            u[0] = up_row[i];
+        }
+#pragma unroll
+        for (int j = 0; j < kWidth; ++j) product[j] = (g[j] / (1.0f + expf(-g[j]))) * u[j];
+        if constexpr (OUT_BF16) {
+            __nv_bfloat16* target = static_cast<__nv_bfloat16*>(out) + member * length + i;
+            if constexpr (VECTOR) {
+                const __nv_bfloat162 low = __floats2bfloat162_rn(product[0], product[1]), high = __floats2bfloat162_rn(product[2], product[3]);
+                *reinterpret_cast<uint2*>(target) = make_uint2(*reinterpret_cast<const uint32_t*>(&low), *reinterpret_cast<const uint32_t*>(&high));
+            } else {
+                *target = __float2bfloat16_rn(product[0]);
+            }
+        } else {
+            float* target = static_cast<float*>(out) + member * length + i;
+            if constexpr (VECTOR) *reinterpret_cast<float4*>(target) = make_float4(product[0], product[1], product[2], product[3]);
+            else *target = product[0];
+        }
     }
 }
 
+// y += x, four values per thread and a scalar tail (both pointers are 16-byte aligned)
 __global__ void __launch_bounds__(256) residual_add_kernel(float* __restrict__ y, const float* __restrict__ x, unsigned long long total) {
     pdl_launch_dependents();
     pdl_wait_prior();   // inputs come from the kernels before this one in the stream
-    for (unsigned long long i = static_cast<unsigned long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
-         i += static_cast<unsigned long long>(gridDim.x) * blockDim.x)
-        y[i] += x[i];
+    const unsigned long long quads = total / 4;
+    const unsigned long long thread = static_cast<unsigned long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+    for (unsigned long long i = thread; i < quads; i += static_cast<unsigned long long>(gridDim.x) * blockDim.x) {
+        const float4 a = reinterpret_cast<const float4*>(y)[i], b = reinterpret_cast<const float4*>(x)[i];
+        reinterpret_cast<float4*>(y)[i] = make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+    }
+    if (thread < total - 4 * quads) y[4 * quads + thread] += x[4 * quads + thread];
 }
 
 // ---------------------------------------------------------------- argmax
-// One CTA per member.  NaN never wins, ties go to the lowest index, a row of NaNs gives 0 -- the reference's
-// rules (model_ops.rs:201-258).  Keys are the monotone unsigned image of the floats.
+// NaN never wins, ties go to the lowest index, a row of NaNs gives 0 -- the reference's rules (model_ops.rs:201-258).
+// A candidate is one 64-bit word: the monotone unsigned image of its value above the complement of its index, so that the
+// largest word is the answer and 0 means "none".
+//
+// Grid (parts, members).  A row is a vocabulary, 128 K values and more, and one CTA reads it at what a single SM can have in
+// flight: 69 us for one row of 151936 values.  Sixteen values per thread and one CTA per 4096 put the whole row in flight at
+// once; the CTAs of a row meet in an atomic maximum and the last to arrive writes the index and leaves the words zero.
+constexpr int kArgmaxThreads = 256;
+constexpr int kArgmaxPerThread = 16;
+constexpr int kArgmaxWordsPerMember = 4;   // of the context's zero-initialised counters: the maximum (two words), arrivals
+
 __device__ __forceinline__ unsigned int logit_key(float value) {
     const unsigned int bits = __float_as_uint(value);
     return (bits >> 31) ? ~bits : (bits ^ 0x80000000u);
 }
 
-__global__ void __launch_bounds__(1024) argmax_kernel(const float* __restrict__ logits, unsigned int* __restrict__ out, unsigned long long length) {
+__global__ void __launch_bounds__(kArgmaxThreads) argmax_kernel(const float* __restrict__ logits, unsigned int* __restrict__ out,
+                                                                unsigned long long length, unsigned int* counters) {
     pdl_launch_dependents();
     pdl_wait_prior();   // inputs come from the kernels before this one in the stream
-    __shared__ unsigned int keys[32];
-    __shared__ unsigned int indices[32];
-    const float* row = logits + static_cast<size_t>(blockIdx.x) * length;
-    unsigned int key = 0u, index = 0u;
-    for (unsigned long long i = threadIdx.x; i < length; i += blockDim.x) {
-        const float candidate = row[i];
-        const unsigned int candidate_key = logit_key(candidate);
-        if (candidate == candidate && candidate_key > key) {
-            key = candidate_key;
-            index = static_cast<unsigned int>(i);
+    __shared__ unsigned long long warp_best[kArgmaxThreads / 32];
+    const float* row = logits + static_cast<size_t>(blockIdx.y) * length;
+    unsigned long long best = 0ull;
+    const unsigned long long stride = static_cast<unsigned long long>(gridDim.x) * (kArgmaxThreads * kArgmaxPerThread);
+    for (unsigned long long first = static_cast<unsigned long long>(blockIdx.x) * (kArgmaxThreads * kArgmaxPerThread) + threadIdx.x; first < length;
+         first += stride) {
+        float value[kArgmaxPerThread];
+#pragma unroll
+        for (int u = 0; u < kArgmaxPerThread; ++u) {
+            const unsigned long long i = first + static_cast<unsigned long long>(u) * kArgmaxThreads;
+            value[u] = i < length ? row[i] : __int_as_float(0x7fc00000);
+        }
+#pragma unroll
+        for (int u = 0; u < kArgmaxPerThread; ++u) {
+            const unsigned int index = static_cast<unsigned int>(first) + static_cast<unsigned int>(u * kArgmaxThreads);
+            const unsigned long long candidate = (static_cast<unsigned long long>(logit_key(value[u])) << 32) | (~index);
+            if (value[u] == value[u] && candidate > best) best = candidate;
         }
     }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-        const unsigned int other_key = __shfl_down_sync(0xffffffffu, key, o);
-        const unsigned int other_index = __shfl_down_sync(0xffffffffu, index, o);
-        if (other_key > key || (other_key == key && other_index < index)) {
-            key = other_key;
-            index = other_index;
-        }
+        const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, o);
+        best = other > best ? other : best;
     }
-    if (lane == 0) {
-        keys[warp] = key;
-        indices[warp] = index;
-    }
+    if ((threadIdx.x & 31) == 0) warp_best[threadIdx.x >> 5] = best;
     __syncthreads();
-    if (warp == 0) {
-        key = lane < static_cast<int>(blockDim.x >> 5) ? keys[lane] : 0u;
-        index = lane < static_cast<int>(blockDim.x >> 5) ? indices[lane] : 0u;
+    if (threadIdx.x != 0) return;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const unsigned int other_key = __shfl_down_sync(0xffffffffu, key, o);
-            const unsigned int other_index = __shfl_down_sync(0xffffffffu, index, o);
-            if (other_key > key || (other_key == key && other_index < index)) {
-                key = other_key;
-                index = other_index;
-            }
-        }
-        if (lane == 0) out[blockIdx.x] = index;
+    for (int w = 1; w < kArgmaxThreads / 32; ++w) best = warp_best[w] > best ? warp_best[w] : best;
+    if (gridDim.x > 1) {
+        unsigned int* words = counters + static_cast<size_t>(blockIdx.y) * kArgmaxWordsPerMember;
+        unsigned long long* maximum = reinterpret_cast<unsigned long long*>(words);
+        if (best != 0ull) atomicMax(maximum, best);
+        __threadfence();
+        if (atomicAdd(words + 2, 1u) != gridDim.x - 1) return;
+        __threadfence();
+        best = atomicExch(maximum, 0ull);   // ready for the next launch
+        words[2] = 0u;
     }
+    out[blockIdx.y] = best == 0ull ? 0u : ~static_cast<unsigned int>(best);
 }
 
 }  // namespace
@@ -496,10 +561,11 @@ cudaError_t launch_embedding(const uint8_t* weights, uint32_t value_type, int k,
 }
 
 cudaError_t launch_qk_norm_rope_append(const LayerAttentionArgs& a) {
-    const dim3 grid(a.q_heads + 2 * a.kv_heads, a.members);
-    return launch_kernel_if(pdl_switch() == 1, qk_norm_rope_append_kernel, grid, dim3(a.head_dim), 0, a.stream, a.q, a.k, a.v, a.q_norm, a.k_norm, a.eps, a.positions,
-                         a.q_heads, a.kv_heads, a.head_dim, a.rot_dims / 2, a.rope_base, static_cast<__half*>(a.k_cache),
-                         static_cast<__half*>(a.v_cache), a.max_context, a.shared_cache ? 1 : 0, a.device_status);
+    if (a.head_dim != kHeadDim) return cudaErrorInvalidValue;
+    const dim3 grid((a.q_heads + 2 * a.kv_heads + kRopeWarps - 1) / kRopeWarps, a.members);
+    return launch_kernel_if(pdl_switch() == 1, qk_norm_rope_append_kernel, grid, dim3(kRopeWarps * 32), 0, a.stream, a.q, a.k, a.v, a.q_norm, a.k_norm,
+                            a.eps, a.positions, a.q_heads, a.kv_heads, a.rot_dims / 2, a.rope_base, static_cast<__half*>(a.k_cache),
+                            static_cast<__half*>(a.v_cache), a.max_context, a.shared_cache ? 1 : 0, a.device_status);
 }
 
 int attention_splits(int members, int kv_heads, long long active_context, int sm_count) {
@@ -519,7 +585,6 @@ size_t attention_scratch_bytes(int members, int q_heads, int splits) {
 
 cudaError_t launch_attention_decode(const LayerAttentionArgs& a, void* out, bool out_bf16, void* scratch, int splits) {
     if (a.head_dim != kAttnHeadDim || a.q_heads % a.kv_heads != 0 || a.q_heads / a.kv_heads > kAttnMaxGroup) return cudaErrorInvalidValue;
-    const int group = a.q_heads / a.kv_heads;
     long long chunk = (a.active_context + splits - 1) / splits;
     chunk = (chunk + kAttnTile - 1) / kAttnTile * kAttnTile;
     float* part_o = static_cast<float*>(scratch);
@@ -547,26 +612,48 @@ cudaError_t launch_attention_decode(const LayerAttentionArgs& a, void* out, bool
 
 cudaError_t launch_silu_mul(const float* gate, const float* up, void* out, bool out_bf16, uint64_t members, uint64_t length, uint64_t in_stride,
                             int sm_count, cudaStream_t stream) {
-    const unsigned long long total = members * length;
-    unsigned long long blocks = (total + 255) / 256;
-    if (blocks > static_cast<unsigned long long>(sm_count) * 8) blocks = static_cast<unsigned long long>(sm_count) * 8;
-    const dim3 grid(static_cast<unsigned>(blocks ? blocks : 1));
-    if (out_bf16)
-        return launch_kernel_if(pdl_switch() == 1, silu_mul_kernel<true>, grid, dim3(256), 0, stream, gate, up, out,
-                                static_cast<unsigned long long>(length), static_cast<unsigned long long>(in_stride), total);
-    return launch_kernel_if(pdl_switch() == 1, silu_mul_kernel<false>, grid, dim3(256), 0, stream, gate, up, out,
-                            static_cast<unsigned long long>(length), static_cast<unsigned long long>(in_stride), total);
+    // rows that all start on 16-byte boundaries: the API checks the pointers, the halves of one row may still be anywhere
+    const bool vector = length % 4 == 0 && in_stride % 4 == 0 && reinterpret_cast<uintptr_t>(gate) % 16 == 0 && reinterpret_cast<uintptr_t>(up) % 16 == 0;
+    const uint64_t per_block = 256 * (vector ? 4 : 1);
+    uint64_t pieces = (length + per_block - 1) / per_block;
+    if (pieces > static_cast<uint64_t>(sm_count) * 8) pieces = static_cast<uint64_t>(sm_count) * 8;
+    auto kernel = out_bf16 ? (vector ? silu_mul_kernel<true, true> : silu_mul_kernel<true, false>)
+                           : (vector ? silu_mul_kernel<false, true> : silu_mul_kernel<false, false>);
+    for (uint64_t first = 0; first < members; first += 65535) {   // members are the grid's y dimension
+        const uint64_t rows = members - first < 65535 ? members - first : 65535;
+        const cudaError_t e = launch_kernel_if(pdl_switch() == 1, kernel, dim3(static_cast<unsigned>(pieces), static_cast<unsigned>(rows)), dim3(256), 0,
+                                               stream, gate, up, out, static_cast<unsigned long long>(length), static_cast<unsigned long long>(in_stride),
+                                               static_cast<unsigned int>(first));
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 cudaError_t launch_residual_add(float* y, const float* x, uint64_t total, int sm_count, cudaStream_t stream) {
-    unsigned long long blocks = (total + 255) / 256;
+    unsigned long long blocks = (total / 4 + 255) / 256;
     if (blocks > static_cast<unsigned long long>(sm_count) * 8) blocks = static_cast<unsigned long long>(sm_count) * 8;
     return launch_kernel_if(pdl_switch() == 1, residual_add_kernel, dim3(static_cast<unsigned>(blocks ? blocks : 1)), dim3(256), 0, stream, y, x,
                          static_cast<unsigned long long>(total));
 }
 
-cudaError_t launch_argmax(const float* logits, int members, uint64_t length, uint32_t* out, cudaStream_t stream) {
-    return launch_kernel_if(pdl_switch() == 1, argmax_kernel, dim3(members), dim3(1024), 0, stream, logits, out, static_cast<unsigned long long>(length));
+cudaError_t launch_argmax(const float* logits, int members, uint64_t length, uint32_t* out, unsigned int* counters, int counter_count, int sm_count,
+                          cudaStream_t stream) {
+    // As many CTAs as the rows have pieces of 4096 values, at most four per SM over all rows; one per row where the counters
+    // do not reach.
+    const uint64_t pieces = (length + kArgmaxThreads * kArgmaxPerThread - 1) / (kArgmaxThreads * kArgmaxPerThread);
+    uint64_t parts = (4ull * sm_count + members - 1) / members;
+    if (parts > pieces) parts = pieces;
+    if (static_cast<int64_t>(members) * kArgmaxWordsPerMember > counter_count) parts = 1;
+    // members is the grid's y dimension
+    if (members <= 0) return cudaErrorInvalidValue;
+    for (int first = 0; first < members; first += 65535) {
+        const int rows = members - first < 65535 ? members - first : 65535;
+        const cudaError_t e = launch_kernel_if(pdl_switch() == 1, argmax_kernel, dim3(static_cast<unsigned>(parts), rows), dim3(kArgmaxThreads), 0, stream,
+                                               logits + static_cast<size_t>(first) * length, out + first, static_cast<unsigned long long>(length),
+                                               counters);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 }  // namespace ribn
