@@ -1299,7 +1299,7 @@ int ribn_attention_decode(ribn_ctx* ctx, const ribn_attention* attention, const 
     if (f.status == RIBN_OK) f = check_device_pointer(ctx, attention->v_cache, "value cache");
     if (f.status != RIBN_OK) return record(ctx, f);
     const ribn::LayerAttentionArgs args = attention_args(ctx, attention, const_cast<float*>(q_device), nullptr, nullptr);
-    int splits = ribn::attention_splits(args.members, args.kv_heads, args.active_context, ctx->sm_count);
+    int splits = ribn::attention_splits(args, ctx->sm_count);
     while (splits > 1 && ribn::attention_scratch_bytes(args.members, args.q_heads, splits) > ctx->workspace_bytes) --splits;
     if (ribn::attention_scratch_bytes(args.members, args.q_heads, splits) > ctx->workspace_bytes)
         return record(ctx, fail(RIBN_E_SHAPE_OVERFLOW, "attention partial results do not fit the context workspace"));

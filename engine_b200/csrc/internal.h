@@ -236,7 +236,7 @@ struct LayerAttentionArgs {
 cudaError_t launch_embedding(const uint8_t* weights, uint32_t value_type, int k, unsigned int vocabulary, const uint32_t* tokens,
                              int members, float* out, cudaStream_t stream);
 cudaError_t launch_qk_norm_rope_append(const LayerAttentionArgs& args);
-int attention_splits(int members, int kv_heads, long long active_context, int sm_count);
+int attention_splits(const LayerAttentionArgs& args, int sm_count);   // 0: the kernel for prompt chunks, which needs no scratch
 size_t attention_scratch_bytes(int members, int q_heads, int splits);
 cudaError_t launch_attention_decode(const LayerAttentionArgs& args, void* out, bool out_bf16, void* scratch, int splits);
 cudaError_t launch_silu_mul(const float* gate, const float* up, void* out, bool out_bf16, uint64_t members, uint64_t length, uint64_t in_stride,

@@ -388,6 +388,210 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 3) attention_split_kernel(con
     }
 }
 
+// ---------------------------------------------------------------- attention of a prompt chunk
+// The members are consecutive tokens of one sequence, so their queries share the keys and values they read.  The kernel above
+// walks the cache once per token with at most eight of the sixteen rows of its MMAs in use (310 us on average for 512 tokens
+// behind 0, 512, 1024 and 1536 others at 32 query and 8 key-value heads).  Here a CTA owns 48 rows = (token, head of the group)
+// pairs of one KV head and one walk serves them all: bound by the MMAs, which are twice as many as a plain f16 product needs
+// because queries and probabilities keep their hi + lo parts.  Warp = (row tile of 16, sixteen tokens of every tile of 64): the
+// same sums in the same order as above, so that a token's result does not depend on which kernel ran.  Three row tiles: twelve
+// warps of 168 registers fill the register file.  Grid (kv_heads, row tiles); the last tokens, which walk furthest, start first.
+constexpr int kChunkRowTiles = 3;
+constexpr int kChunkRows = 16 * kChunkRowTiles;
+constexpr int kChunkWarps = kAttnWarps * kChunkRowTiles;
+constexpr int kChunkMergeBytes = kAttnWarps * kChunkRows * (kAttnHeadDim + 2) * 4;
+constexpr int kChunkSmemBytes = kAttnSmemBytes > kChunkMergeBytes ? kAttnSmemBytes : kChunkMergeBytes;
+
+template <bool OUT_BF16>
+__global__ void __launch_bounds__(kChunkWarps * 32, 1) attention_chunk_kernel(const float* __restrict__ q, const __half* __restrict__ k_cache,
+                                                                              const __half* __restrict__ v_cache, const int* __restrict__ positions,
+                                                                              void* __restrict__ out, int members, int q_heads, int kv_heads,
+                                                                              long long max_context, float scale, int active_context,
+                                                                              int* __restrict__ status) {
+    pdl_launch_dependents();
+    pdl_wait_prior();   // inputs come from the kernels before this one in the stream
+    extern __shared__ __align__(128) uint8_t attn_smem[];
+    __shared__ int warp_limit[kChunkWarps];
+    const int kv_head = blockIdx.x;
+    const int group = q_heads / kv_heads;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int tile = warp / kAttnWarps, part = warp % kAttnWarps;   // row tile; which sixteen tokens of every 64
+    const int g = lane >> 2, t = lane & 3;
+    const int cta_row = static_cast<int>(gridDim.y - 1 - blockIdx.y) * kChunkRows;   // of members * group rows of this KV head
+
+    // Tokens each of this thread's two rows may look at; positions[] is device memory: clamped and reported like above.
+    int limit[2];
+    const float* q_row[2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const int row = cta_row + tile * 16 + g + 8 * r;
+        const int member = row / group;
+        limit[r] = 0;
+        q_row[r] = nullptr;
+        if (member < members) {
+            limit[r] = positions[member] + 1;
+            if (limit[r] < 1 || limit[r] > active_context) {
+                if (t == 0) atomicExch(status, kDevicePositionOutOfRange);
+                limit[r] = max(0, min(limit[r], active_context));
+            }
+            q_row[r] = q + (static_cast<size_t>(member) * q_heads + static_cast<size_t>(kv_head) * group + (row - member * group)) * kAttnHeadDim;
+        }
+    }
+    const int tile_end = __reduce_max_sync(0xffffffffu, max(limit[0], limit[1]));
+    if (lane == 0) warp_limit[warp] = tile_end;
+    __syncthreads();
+    int end = 0;
+#pragma unroll
+    for (int w = 0; w < kChunkWarps; ++w) end = max(end, warp_limit[w]);
+
+    const __half* k_base = k_cache + static_cast<long long>(kv_head) * max_context * kAttnHeadDim;
+    const __half* v_base = v_cache + static_cast<long long>(kv_head) * max_context * kAttnHeadDim;
+    const uint32_t smem_base = static_cast<uint32_t>(__cvta_generic_to_shared(attn_smem));
+    auto request_tile = [&](int buffer, int t0) {
+        const int valid = min(kAttnTile, end - t0);
+        for (int i = threadIdx.x; i < kAttnTile * (kAttnHeadDim / 8); i += kChunkWarps * 32) {
+            const int row = i / (kAttnHeadDim / 8);
+            const int piece = i % (kAttnHeadDim / 8);
+            const uint32_t kd = smem_base + (2 * buffer) * kAttnTileBytes + (row * kAttnKStride + 8 * piece) * 2;
+            const uint32_t vd = kd + kAttnTileBytes;
+            if (row < valid) {
+                const __half* ks = k_base + static_cast<long long>(t0 + row) * kAttnHeadDim + 8 * piece;
+                const __half* vs = v_base + static_cast<long long>(t0 + row) * kAttnHeadDim + 8 * piece;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(kd), "l"(ks) : "memory");
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(vd), "l"(vs) : "memory");
+            } else {
+                asm volatile("st.shared.v4.b32 [%0], {%1,%1,%1,%1};" ::"r"(kd), "r"(0) : "memory");
+                asm volatile("st.shared.v4.b32 [%0], {%1,%1,%1,%1};" ::"r"(vd), "r"(0) : "memory");
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if (end > 0) request_tile(0, 0);   // in flight while the queries are fetched and split below
+
+    uint32_t q_hi[8][4], q_lo[8][4];
+    {
+        const float factor = scale * 1.4426950408889634f;
+#pragma unroll
+        for (int ks = 0; ks < 8; ++ks) {
+#pragma unroll
+            for (int piece = 0; piece < 4; ++piece) {
+                float2 v = make_float2(0.0f, 0.0f);
+                if (q_row[piece & 1] != nullptr) v = *reinterpret_cast<const float2*>(q_row[piece & 1] + 16 * ks + 2 * t + 8 * (piece >> 1));
+                split_half2(v.x * factor, v.y * factor, q_hi[ks][piece], q_lo[ks][piece]);
+            }
+        }
+    }
+    float acc[16][4];   // rows g, g + 8; dims 8 n + 2 t, + 1
+#pragma unroll
+    for (int n = 0; n < 16; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.0f;
+    float running_max[2] = {-INFINITY, -INFINITY}, running_sum[2] = {0.0f, 0.0f};
+    const uint32_t k_lane = ((16 * part + (lane & 7) + 8 * (lane >> 4)) * kAttnKStride + 8 * ((lane >> 3) & 1)) * 2;
+    const uint32_t v_lane = ((16 * part + (lane & 7) + 8 * ((lane >> 3) & 1)) * kAttnKStride + 8 * (lane >> 4)) * 2;
+
+    int buffer = 0;
+    for (int t0 = 0; t0 < end; t0 += kAttnTile, buffer ^= 1) {
+        if (t0 + kAttnTile < end) {
+            request_tile(buffer ^ 1, t0 + kAttnTile);   // its previous contents were consumed before the barrier that ended the last round
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();   // this tile has landed for every thread
+        const int first = t0 + 16 * part;
+        if (first < tile_end) {
+            const uint32_t k_tile = smem_base + (2 * buffer) * kAttnTileBytes, v_tile = k_tile + kAttnTileBytes;
+            float s[2][4] = {{0.0f, 0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f, 0.0f}};
+#pragma unroll
+            for (int ks = 0; ks < 8; ++ks) {
+                uint32_t b[4];
+                ldmatrix_x4(k_tile + k_lane + 32 * ks, b);
+                mma_f16(s[0], q_hi[ks], b[0], b[1]);
+                mma_f16(s[1], q_hi[ks], b[2], b[3]);
+                mma_f16(s[0], q_lo[ks], b[0], b[1]);
+                mma_f16(s[1], q_lo[ks], b[2], b[3]);
+            }
+            uint32_t p_hi[4], p_lo[4];
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+#pragma unroll
+                for (int n = 0; n < 2; ++n) {
+#pragma unroll
+                    for (int c = 2 * r; c < 2 * r + 2; ++c)
+                        if (first + 8 * n + 2 * t + (c & 1) >= limit[r]) s[n][c] = -INFINITY;
+                }
+                float tile_max = fmaxf(fmaxf(s[0][2 * r], s[0][2 * r + 1]), fmaxf(s[1][2 * r], s[1][2 * r + 1]));
+                tile_max = fmaxf(tile_max, __shfl_xor_sync(0xffffffffu, tile_max, 1));
+                tile_max = fmaxf(tile_max, __shfl_xor_sync(0xffffffffu, tile_max, 2));
+                const float new_max = fmaxf(running_max[r], tile_max);
+                const float shift = new_max == -INFINITY ? 0.0f : new_max;   // a row that sees none of these tokens
+                const bool moved = new_max != running_max[r];
+                const float rescale = exp2f(running_max[r] - shift);          // 0 the first time round
+                running_max[r] = new_max;
+                const float p0 = exp2f(s[0][2 * r] - shift), p1 = exp2f(s[0][2 * r + 1] - shift);
+                const float p2 = exp2f(s[1][2 * r] - shift), p3 = exp2f(s[1][2 * r + 1] - shift);
+                running_sum[r] = running_sum[r] * rescale + ((p0 + p1) + (p2 + p3));   // this lane's share; lanes are added at the end
+                if (__any_sync(0xffffffffu, moved)) {   // rare after the first tiles; the factor is one otherwise
+#pragma unroll
+                    for (int n = 0; n < 16; ++n) {
+                        acc[n][2 * r] *= rescale;
+                        acc[n][2 * r + 1] *= rescale;
+                    }
+                }
+                split_half2(p0, p1, p_hi[r], p_lo[r]);
+                split_half2(p2, p3, p_hi[2 + r], p_lo[2 + r]);
+            }
+#pragma unroll
+            for (int pair = 0; pair < 8; ++pair) {
+                uint32_t b[4];
+                ldmatrix_x4_trans(v_tile + v_lane + 32 * pair, b);
+                mma_f16(acc[2 * pair], p_hi, b[0], b[1]);
+                mma_f16(acc[2 * pair + 1], p_hi, b[2], b[3]);
+                mma_f16(acc[2 * pair], p_lo, b[0], b[1]);
+                mma_f16(acc[2 * pair + 1], p_lo, b[2], b[3]);
+            }
+        }
+        __syncthreads();   // every warp is done with this buffer before the next round refills it
+    }
+
+    // merge the four token parts: [part][row] maximum and sum, [part][row][dim] output, in the tile buffers
+    float* merge_o = reinterpret_cast<float*>(attn_smem);                    // [4][48][128]
+    float* merge_m = merge_o + kAttnWarps * kChunkRows * kAttnHeadDim;        // [4][48]
+    float* merge_l = merge_m + kAttnWarps * kChunkRows;
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        running_sum[r] += __shfl_xor_sync(0xffffffffu, running_sum[r], 1);
+        running_sum[r] += __shfl_xor_sync(0xffffffffu, running_sum[r], 2);
+        const int row = part * kChunkRows + tile * 16 + g + 8 * r;
+        if (t == 0) {
+            merge_m[row] = running_max[r];
+            merge_l[row] = running_sum[r];
+        }
+#pragma unroll
+        for (int n = 0; n < 16; ++n)
+            *reinterpret_cast<float2*>(merge_o + row * kAttnHeadDim + 8 * n + 2 * t) = make_float2(acc[n][2 * r], acc[n][2 * r + 1]);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < kChunkRows * kAttnHeadDim; i += kChunkWarps * 32) {
+        const int row = i / kAttnHeadDim, dim = i % kAttnHeadDim;
+        const int member = (cta_row + row) / group;
+        if (member >= members) break;
+        float top = -INFINITY;
+#pragma unroll
+        for (int w = 0; w < kAttnWarps; ++w) top = fmaxf(top, merge_m[w * kChunkRows + row]);
+        float total = 0.0f, value = 0.0f;
+#pragma unroll
+        for (int w = 0; w < kAttnWarps; ++w) {
+            const float m = merge_m[w * kChunkRows + row];
+            const float weight = m == -INFINITY ? 0.0f : exp2f(m - top);
+            total = fmaf(merge_l[w * kChunkRows + row], weight, total);
+            value = fmaf(merge_o[(w * kChunkRows + row) * kAttnHeadDim + dim], weight, value);
+        }
+        const size_t index = (static_cast<size_t>(member) * q_heads + static_cast<size_t>(kv_head) * group + (cta_row + row - member * group)) * kAttnHeadDim + dim;
+        if constexpr (OUT_BF16) static_cast<__nv_bfloat16*>(out)[index] = __float2bfloat16_rn(value / total);
+        else static_cast<float*>(out)[index] = value / total;
+    }
+}
+
 // grid (q_heads, members), 128 threads: merges the splits of one query head.  Lane s of every warp holds split s (at most 32
 // splits): the maximum, the sum and the weights come out of two warp reductions, and a thread then has sixteen partial rows
 // of its output dimension in flight at a time.
@@ -568,13 +772,22 @@ cudaError_t launch_qk_norm_rope_append(const LayerAttentionArgs& a) {
                             static_cast<__half*>(a.v_cache), a.max_context, a.shared_cache ? 1 : 0, a.device_status);
 }
 
-int attention_splits(int members, int kv_heads, long long active_context, int sm_count) {
+// Consecutive tokens of one sequence go to the chunk kernel once the token-by-token walk has enough CTAs to leave the context
+// unsplit (four per SM) and the chunk's row tiles occupy at least half of the SMs; below that the walk, spread over the SMs, is
+// the faster one.
+static bool attention_is_chunk(const LayerAttentionArgs& a, int sm_count) {
+    const long long tiles = (static_cast<long long>(a.members) * (a.q_heads / a.kv_heads) + kChunkRows - 1) / kChunkRows;
+    return a.shared_cache && static_cast<long long>(a.members) * a.kv_heads > 4ll * sm_count && 2 * tiles * a.kv_heads >= sm_count;
+}
+
+int attention_splits(const LayerAttentionArgs& a, int sm_count) {
+    if (attention_is_chunk(a, sm_count)) return 0;   // no partial results
     // About eight CTAs per SM: a CTA walks its tiles one after the other, so the memory latency is hidden by
     // the CTAs that share its SM.
-    int splits = (8 * sm_count) / (members * kv_heads);
+    int splits = (8 * sm_count) / (a.members * a.kv_heads);
     if (splits < 1) splits = 1;
     if (splits > 32) splits = 32;
-    const long long tiles = (active_context + kAttnTile - 1) / kAttnTile;
+    const long long tiles = (a.active_context + kAttnTile - 1) / kAttnTile;
     if (splits > tiles) splits = static_cast<int>(tiles < 1 ? 1 : tiles);
     return splits;
 }
@@ -583,8 +796,28 @@ size_t attention_scratch_bytes(int members, int q_heads, int splits) {
     return static_cast<size_t>(members) * q_heads * splits * (kAttnHeadDim + 2) * sizeof(float);
 }
 
+static cudaError_t launch_attention_chunk(const LayerAttentionArgs& a, void* out, bool out_bf16) {
+    const float scale = 1.0f / sqrtf(static_cast<float>(a.head_dim));
+    auto kernel = out_bf16 ? attention_chunk_kernel<true> : attention_chunk_kernel<false>;
+    static int configured_device = -1;
+    int device = 0;
+    cudaGetDevice(&device);
+    if (configured_device != device) {
+        cudaError_t attribute = cudaFuncSetAttribute(attention_chunk_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kChunkSmemBytes);
+        if (attribute == cudaSuccess)
+            attribute = cudaFuncSetAttribute(attention_chunk_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kChunkSmemBytes);
+        if (attribute != cudaSuccess) return attribute;
+        configured_device = device;
+    }
+    const int tiles = (a.members * (a.q_heads / a.kv_heads) + kChunkRows - 1) / kChunkRows;
+    return launch_kernel_if(pdl_switch() == 1, kernel, dim3(a.kv_heads, tiles), dim3(kChunkWarps * 32), kChunkSmemBytes, a.stream,
+                            static_cast<const float*>(a.q), static_cast<const __half*>(a.k_cache), static_cast<const __half*>(a.v_cache), a.positions, out,
+                            a.members, a.q_heads, a.kv_heads, a.max_context, scale, static_cast<int>(a.active_context), a.device_status);
+}
+
 cudaError_t launch_attention_decode(const LayerAttentionArgs& a, void* out, bool out_bf16, void* scratch, int splits) {
     if (a.head_dim != kAttnHeadDim || a.q_heads % a.kv_heads != 0 || a.q_heads / a.kv_heads > kAttnMaxGroup) return cudaErrorInvalidValue;
+    if (splits == 0) return launch_attention_chunk(a, out, out_bf16);
     long long chunk = (a.active_context + splits - 1) / splits;
     chunk = (chunk + kAttnTile - 1) / kAttnTile * kAttnTile;
     float* part_o = static_cast<float*>(scratch);
