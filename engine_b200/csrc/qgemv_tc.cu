@@ -9,8 +9,7 @@
 //
 // A tcgen05.mma of 128 rows x 16 K costs the pipe about 54 cycles however few tokens it has (measured
 // for N <= 64), so the number of MMAs per weight decides the ceiling: this kernel issues one per 16 K
-// elements (the dequantised-operand GEMM of qgemm_tc.cu, which splits every weight into two bf16
-// parts, needs two), and it keeps the per-weight ALU work to the dequantisation itself.
+// elements, and it keeps the per-weight ALU work to the dequantisation itself.
 //
 // Operand encoding.  f16 has 11 significant bits (2^-12 relative rounding, inside the 2e-3 bound of
 // the path; a bf16 tile would not be) but only five exponent bits.  Range is handled exactly:

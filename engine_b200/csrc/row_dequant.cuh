@@ -23,42 +23,11 @@ __device__ __forceinline__ uint4 raw16_a2(const uint8_t* p) {
     return v;
 }
 
-// Operand encodings.  An encoder turns eight f32 weights into one 16-byte chunk of a K-major tile
-// (or one chunk per plane).
+// Operand encodings.  An encoder turns eight f32 weights into one 16-byte chunk of a K-major tile.
 //
-// SplitBf16: w_high = bf16(w) and w_low = bf16(w - w_high), two tiles, together 16 significant bits.
-struct SplitBf16 {
-    static constexpr bool kFoldOffset = false;   // 16 significant bits: keep the exact two-step dequantisation
-    struct Chunk {
-        uint4 high, low;
-    };
-    __device__ static void pair(float w0, float w1, uint32_t& high, uint32_t& low) {
-        const __nv_bfloat162 h = __floats2bfloat162_rn(w0, w1);
-        high = *reinterpret_cast<const uint32_t*>(&h);
-        const float h0 = __uint_as_float(high << 16);
-        const float h1 = __uint_as_float(high & 0xffff0000u);
-        const __nv_bfloat162 l = __floats2bfloat162_rn(w0 - h0, w1 - h1);
-        low = *reinterpret_cast<const uint32_t*>(&l);
-    }
-    __device__ static Chunk encode(const float (&a)[4], const float (&b)[4]) {
-        Chunk out;
-        pair(a[0], a[1], out.high.x, out.low.x);
-        pair(a[2], a[3], out.high.y, out.low.y);
-        pair(b[0], b[1], out.high.z, out.low.z);
-        pair(b[2], b[3], out.high.w, out.low.w);
-        return out;
-    }
-    __device__ static Chunk zero() {
-        Chunk out;
-        out.high = out.low = make_uint4(0, 0, 0, 0);
-        return out;
-    }
-};
-
 // SingleF16: one f16 tile (11 significant bits); the caller keeps the values in f16 range by
 // pre-scaling each super-block (see RowDequant::magnitude_bound).
 struct SingleF16 {
-    static constexpr bool kFoldOffset = true;
     struct Chunk {
         uint4 high;
     };
@@ -88,7 +57,7 @@ __device__ __forceinline__ float byte_plus_128(uint32_t packed) {
 template <class Enc>
 __device__ __forceinline__ typename Enc::Chunk chunk_from_bytes(uint32_t q0, uint32_t q1, float bias, float scale, float minimum) {
     float a[4], b[4];
-    if (Enc::kFoldOffset && bias < 100.0f) {
+    if (bias < 100.0f) {
         // Quants below 128 (every K-quant): w = scale * (128 + q) - (scale * (128 + bias) + minimum), one prmt and one
         // FMA per weight.  The folded constant is rounded at the magnitude of 160 * scale, 2^-17 of a quant step: far
         // below the f16 rounding that follows (the exact two-step form is kept where results must be bit-exact).

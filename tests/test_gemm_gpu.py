@@ -154,3 +154,27 @@ def test_rejections_leave_output_untouched(ctx):
                                          torch.zeros((2, 4), device=ctx.device))) == "InvalidWeight"
     ctx.synchronize()
     assert torch.all(y == 7.0)
+
+
+# the edges of the prompt kernel's work split: two sums and split-K (few rows), one sum over several units per pair of SMs (many
+# rows), ragged rows and tokens, rows that do not start on 16-byte boundaries; against the exactly dequantised weights in f64
+@pytest.mark.parametrize("vt,n,k,m", [(12, 130, 256, 65), (14, 2000, 1280, 129), (13, 4100, 768, 257), (8, 9000, 512, 400), (12, 15300, 512, 300),
+                                      (14, 15300, 1280, 513), (13, 16384, 256, 1000), (12, 640, 4096, 173)])
+@pytest.mark.parametrize("y_dtype", [torch.float32, torch.bfloat16])
+def test_prompt_kernel_edges(ctx, vt, n, k, m, y_dtype):
+    weight = upload(ctx, vt, synth.random_weight(vt, k, n, seed=n + m), k, n)
+    generator = torch.Generator(device=ctx.device)
+    generator.manual_seed(m)
+    x = torch.randn(m, k, device=ctx.device, generator=generator).to(torch.bfloat16)
+    y = torch.full((m, n), float("nan"), dtype=y_dtype, device=ctx.device)
+    again = torch.empty_like(y)
+    exact = torch.empty(n, k, device=ctx.device)
+    engine_b200.dequantize(ctx, weight, exact)
+    engine_b200.gemm(ctx, weight, x, y)
+    engine_b200.gemm(ctx, weight, x, again)
+    ctx.synchronize()
+    expected = x.double() @ exact.double().T
+    scale = torch.sqrt(x.double().square() @ exact.double().square().T)
+    bound = (TOL + (BF16_ROUNDOFF if y_dtype == torch.bfloat16 else 0.0)) * torch.maximum(expected.abs(), scale)
+    assert torch.all((y.double() - expected).abs() <= bound)
+    assert torch.equal(y, again), "results do not depend on the order in which CTAs arrive"
