@@ -360,12 +360,20 @@ int enqueue_tmem(ribn_ctx* ctx, const ribn_qweight* w, uint64_t k, uint64_t n, c
     return RIBN_OK;
 }
 
+// The integer tensor-core kernel, eight member rows per launch (quants go to the instruction as 8-bit operands).
+bool imma_serves(const ribn_ctx* ctx, const ribn_qweight* w, uint64_t k, uint64_t n, uint32_t members) {
+    const int per_launch = members < 8 ? static_cast<int>(members) : 8;
+    return ctx->imma_gemv != 0 && (members <= static_cast<uint32_t>(ctx->imma_max_members) || members > 8) &&
+           ribn::gemv_imma_supports(w->value_type, static_cast<int>(k), static_cast<int>(n), per_launch, w->data);
+}
+
 // The half2-unpack + mma.sync kernel, eight member rows per launch.  mode: 0 plain, 1 RMSNorm, 2 silu(gate) * up.
 // `image_ready` = the activation images of this x are already in the workspace (an earlier projection of the
 // same fused call made them).
 bool mma_serves(const ribn_ctx* ctx, const ribn_qweight* w, uint64_t k, uint64_t n, uint32_t members) {
     if (ctx->mma_gemv == 0 || ctx->gemv_path != 0) return false;
     const int per_launch = members < 8 ? static_cast<int>(members) : 8;
+    if (imma_serves(ctx, w, k, n, members)) return true;
     return ribn::gemv_mma_supports(w->value_type, static_cast<int>(k), static_cast<int>(n), per_launch, w->data);
 }
 
@@ -377,12 +385,14 @@ int enqueue_mma(ribn_ctx* ctx, const ribn_qweight* w, uint64_t k, uint64_t n, co
     const uint64_t x_row_bytes = k * (mode == 2 ? 2 : 1) * dtype_bytes(x_dtype);
     unsigned none_made = 0;
     if (images_made == nullptr) images_made = &none_made;
-    // The integer tensor-core kernel, eight rows per launch (quants go to the instruction as 8-bit operands).
     const uint32_t per_launch = members < 8 ? members : 8;
-    if (ctx->imma_gemv != 0 && (members <= static_cast<uint32_t>(ctx->imma_max_members) || members > 8) &&
-        ribn::gemv_imma_supports(w->value_type, static_cast<int>(k), static_cast<int>(n), static_cast<int>(per_launch), w->data)) {
+    if (imma_serves(ctx, w, k, n, members)) {
         // its images follow the ones the f16 kernel would keep for the same call
         uint64_t offset = static_cast<uint64_t>((members + 7) / 8) * ribn::gemv_mma_image_bytes(static_cast<int>(per_launch), static_cast<int>(k), 2);
+        // Q8_0 rows may keep their images in an order of their own, behind the plain ones
+        const bool rotated = ribn::gemv_imma_rotates(w->value_type, static_cast<int>(k));
+        const unsigned made = rotated ? 4u : 2u;
+        if (rotated) offset += static_cast<uint64_t>((members + 7) / 8) * ribn::gemv_imma_image_bytes(static_cast<int>(per_launch), static_cast<int>(k));
         for (uint32_t m0 = 0; m0 < members; m0 += 8) {
             ribn::MmaGemvArgs a{};
             a.weights = static_cast<const uint8_t*>(w->data);
@@ -410,7 +420,7 @@ int enqueue_mma(ribn_ctx* ctx, const ribn_qweight* w, uint64_t k, uint64_t n, co
             if (wide && offset + image_bytes <= ctx->workspace_bytes) {
                 void* image = static_cast<uint8_t*>(ctx->workspace) + offset;
                 offset += image_bytes;
-                if ((*images_made & 2u) == 0) {
+                if ((*images_made & made) == 0) {
                     const cudaError_t e = ribn::launch_gemv_imma_image(a, image);
                     if (e != cudaSuccess) return record_cuda(ctx, e, "activation image launch");
                 }
@@ -419,7 +429,7 @@ int enqueue_mma(ribn_ctx* ctx, const ribn_qweight* w, uint64_t k, uint64_t n, co
             const cudaError_t e = ribn::launch_gemv_imma(a);
             if (e != cudaSuccess) return record_cuda(ctx, e, "GEMV launch");
         }
-        *images_made |= 2u;
+        *images_made |= made;
         return RIBN_OK;
     }
     const bool image_ready = (*images_made & 1u) != 0;

@@ -45,28 +45,43 @@
 namespace ribn {
 namespace {
 
-constexpr int kWarps = 8;                      // consumer warps = super-blocks per stage
-constexpr int kConsumers = kWarps * 32;
+constexpr int kGroupWarps = 8;                 // warps of a consumer group = super-blocks per stage
+constexpr int kGroups = 2;                     // consumer groups of a CTA
+constexpr int kConsumerWarps = kGroups * kGroupWarps;
+constexpr int kConsumers = kConsumerWarps * 32;
 constexpr int kThreads = kConsumers + 32;      // + the producer warp
 constexpr int kTileRows = 16;                  // weight rows per tile (the M of m16n8k32)
 constexpr int kMaxStages = 8;
+constexpr int kMaxSlots = 5;                   // tiles of a group whose partial sums may be waiting for their finisher
 constexpr int kMaxMembers = 8;                 // four column groups of two members
 constexpr int kSliceBytes = 768;               // image bytes per (member, super-block): 8 sub-blocks x 3 planes x 32
 constexpr int kZeroBytes = 1024;               // zeros the fourth column of every member (and absent members) read
 
-template <uint32_t FMT>
+// How the weight rows reach shared memory.
+//   kBoxes: tiled TMA, every row on a 16-byte boundary;
+//   kRowsEven: one bulk copy per row and box from the boundary below (Q6_K rows of an even number of super-blocks start on a
+//          word, so whether a super-block starts on a word is the same for all rows);
+//   kRowsOdd: the same for rows that start two bytes off a word in some lanes and on it in others.
+enum Fetch { kBoxes = 0, kRowsEven = 1, kRowsOdd = 2 };
+
+template <uint32_t FMT, int FETCH>
 struct ImmaPlan {
+    // bytes of 256 weights: one super-block, or eight blocks of Q8_0
     static constexpr int kSbBytes = Format<FMT>::kBytes;
-    // Super-blocks per TMA box.  Q4_K / Q5_K: two, a row pitch of 288 / 352 bytes = 8 or 24 (mod 32) words, so that the
-    // 64-bit loads of four rows x four lanes fall on 32 different banks.  Q6_K: eight (1680 bytes, the smallest multiple of
-    // 210 that is a multiple of 16) = 4 (mod 32) words: the 32-bit loads of eight rows x four lanes fall on 32 banks.
-    static constexpr int kBoxSb = FMT == kQ6_K ? 8 : 2;
-    static constexpr int kBoxes = kWarps / kBoxSb;
-    static constexpr int kRowPitch = kBoxSb * kSbBytes;
+    // Super-blocks per box, and bytes from one row of a box to the next (in 4-byte words, mod 32, below): long rows, because the
+    // copy engine works in rows, and a pitch that spreads a warp's loads over the banks.  Q4_K / Q5_K: eight, 1184 / 1440
+    // bytes = 8 words, so that the 64-bit loads of four rows x four lanes fall on 32 different banks.  Q6_K: eight, 1680
+    // bytes = 4, or 1712 = 12 with room for a row that starts up to 14 bytes behind the boundary its copy starts at; Q8_0:
+    // four, 1104 = 20: the 32-bit loads of eight rows x four lanes on 32 banks.
+    static constexpr int kBoxSb = FMT == kQ8_0 ? 4 : 8;
+    static constexpr int kBoxesPerStage = kGroupWarps / kBoxSb;
+    static constexpr int kBoxSpan = kBoxSb * kSbBytes;   // bytes of a row from one box to the next
+    static constexpr int kRowPitch = FMT == kQ8_0 ? kBoxSpan + 16 : FMT == kQ6_K && FETCH == kBoxes ? kBoxSpan : kBoxSpan + 32;
     static constexpr int kBoxBytes = kTileRows * kRowPitch;
-    static constexpr int kStageBytes = kBoxes * kBoxBytes;
-    static_assert(kRowPitch % 16 == 0 && kBoxBytes % 128 == 0, "TMA box: 16-byte rows, 128-byte aligned destination");
-    static_assert((kSbBytes * kBoxSb / 8) % 2 == 0, "TMA x coordinate of every box on a 16-byte boundary");
+    static constexpr int kStageBytes = kBoxesPerStage * kBoxBytes;
+    static_assert(kRowPitch % 16 == 0 && kBoxBytes % 128 == 0, "box: 16-byte rows, 128-byte aligned destination");
+    static_assert(kBoxSpan % 16 == 0, "every box of a row starts as far from a 16-byte boundary as the row does");
+    static_assert(FETCH == kBoxes || FMT == kQ6_K || FMT == kQ8_0, "rows of the other formats are multiples of 16 bytes");
 };
 
 struct ImmaParams {
@@ -76,10 +91,15 @@ struct ImmaParams {
     const float* norm_weight;
     float eps;
     const uint8_t* image;       // activation image made by the pre-pass (layout below), or null: convert here
+    int rotated;                // Q8_0 in boxes: even blocks of the image start at their third element
+    const uint8_t* weights;
+    unsigned long long row_bytes, weight_bytes;
     void* y;
     int y_bf16;
     int accumulate;
     int k, n, nsb, members, stages;
+    int slots;                  // partial-sum slots per consumer group
+    int tile_quotient, tile_remainder;   // tiles per CTA, and how many CTAs have one more
     int* status;
 };
 
@@ -87,7 +107,8 @@ struct ImmaParams {
 // Per call, in shared memory (and in global memory when a pre-pass makes it):
 //   planes [members][nsb][8 sub-blocks][p0 32 B | p1 32 B | p2 32 B] int8, bytes in element order.  The 64-bit
 //          fragment loads of a half-warp (one member: three planes and the zero column, four lanes each) then
-//          cover 96 contiguous bytes plus 32 bytes of the zero area placed 96 bytes further on: 32 banks;
+//          cover 96 contiguous bytes plus 32 bytes of the zero area placed 96 bytes further on: 32 banks.
+//          Rotated (Q8_0 blocks fetched in boxes): blocks 0, 2, 4, 6 hold elements 2 .. 31, 0, 1 -- see superblock_q8;
 //   sums   [members][nsb][16] f16: (sum of the sub-block's 32 integers) / 2^11 as f16 hi (8 values) then f16 lo (8);
 //   scale  [nsb][8] f32: 2^-e per (super-block, member), 0 for an all-zero slice, NaN when it holds a non-finite value.
 __host__ __device__ inline size_t image_plane_bytes(int members, int nsb) { return static_cast<size_t>(members) * nsb * kSliceBytes; }
@@ -97,27 +118,35 @@ __host__ __device__ inline size_t image_bytes(int members, int nsb) {
     return image_plane_bytes(members, nsb) + image_sums_bytes(members, nsb) + image_scale_bytes(nsb);
 }
 
-// Lane `lane` of a warp loads elements 8 lane .. 8 lane + 7 of super-block sb of member row m, prologue applied.
-__device__ __forceinline__ void load_slice(const ImmaParams& p, int m, int sb, int lane, float inv_rms, float (&v)[8]) {
-    const int k0 = sb * kSuperBlock + lane * 8;
+__device__ __forceinline__ AnyRow member_row(const ImmaParams& p, int m) {
     const size_t row_elements = static_cast<size_t>(p.k) * (p.mode == 2 ? 2 : 1);
-    const AnyRow row{static_cast<const uint8_t*>(p.x) + static_cast<size_t>(m) * row_elements * (p.x_bf16 ? 2 : 4), p.x_bf16};
+    return AnyRow{static_cast<const uint8_t*>(p.x) + static_cast<size_t>(m) * row_elements * (p.x_bf16 ? 2 : 4), p.x_bf16};
+}
+
+// Lane `lane` of a warp loads elements 8 lane .. 8 lane + 7 of super-block sb (zeros behind the end of a row), and what the
+// prologue multiplies them by: the norm weights (mode 1) or the row's second half (mode 2).
+__device__ __forceinline__ void load_slice(const ImmaParams& p, int m, int sb, int lane, float (&v)[8], float (&by)[8]) {
+    const int k0 = sb * kSuperBlock + lane * 8;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = 0.0f;
+    if (k0 >= p.k) return;
+    const AnyRow row = member_row(p, m);
     load_row8(row + k0, v);
-    if (p.mode == 2) {
-        float u[8];
-        load_row8(row + (p.k + k0), u);
+    if (p.mode != 0) load_row8(p.mode == 1 ? AnyRow{reinterpret_cast<const uint8_t*>(p.norm_weight), 0} + k0 : row + (p.k + k0), by);
+}
+// The prologue: x * inv_rms * norm weight, or silu(gate) * up.
+__device__ __forceinline__ void apply_prologue(const ImmaParams& p, float inv_rms, float (&v)[8], const float (&by)[8]) {
+    if (p.mode == 1) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = (v[j] / (1.0f + expf(-v[j]))) * u[j];
-    } else if (p.mode == 1) {
-        float g[8];
-        load_x8<float>(p.norm_weight + k0, g);
+        for (int j = 0; j < 8; ++j) v[j] = v[j] * inv_rms * by[j];
+    } else if (p.mode == 2) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = v[j] * inv_rms * g[j];
+        for (int j = 0; j < 8; ++j) v[j] = (v[j] / (1.0f + expf(-v[j]))) * by[j];
     }
 }
 
 // The warp's 256 values -> three int8 planes, block sums and the slice's factor (generic pointers: shared or global).
-__device__ __forceinline__ void store_slice(int m, int sb, int lane, float (&v)[8], uint8_t* planes_row, __half* sums_row, float* scale) {
+__device__ __forceinline__ void store_slice(bool rotated, int m, int sb, int lane, float (&v)[8], uint8_t* planes_row, __half* sums_row, float* scale) {
     // Largest magnitude in one warp reduction: non-negative floats order like their bit patterns, and infinities
     // and NaNs (0x7f800000 and above) come out on top, which is how they are detected.
     uint32_t biggest = 0u;
@@ -146,6 +175,17 @@ __device__ __forceinline__ void store_slice(int m, int sb, int lane, float (&v)[
     sum += __shfl_xor_sync(0xffffffffu, sum, 1);
     sum += __shfl_xor_sync(0xffffffffu, sum, 2);
     const int j = lane >> 2, t = lane & 3;
+    if (rotated) {
+        // even blocks move by two elements: the lane's last two come from the next lane of the block
+        const int next = (lane & ~3) | ((lane + 1) & 3);
+        const int n0 = __shfl_sync(0xffffffffu, xi[0], next), n1 = __shfl_sync(0xffffffffu, xi[1], next);
+        if ((j & 1) == 0) {
+#pragma unroll
+            for (int i = 0; i < 6; ++i) xi[i] = xi[i + 2];
+            xi[6] = n0;
+            xi[7] = n1;
+        }
+    }
     uint8_t* slot = planes_row + static_cast<size_t>(sb) * kSliceBytes + j * 96 + 8 * t;
     *reinterpret_cast<uint2*>(slot) = make_uint2(pack4(xi[0] & 127, xi[1] & 127, xi[2] & 127, xi[3] & 127),
                                                  pack4(xi[4] & 127, xi[5] & 127, xi[6] & 127, xi[7] & 127));
@@ -164,8 +204,9 @@ __device__ __forceinline__ void store_slice(int m, int sb, int lane, float (&v)[
 
 // sum of squares of member row m over the whole K range, by `threads` threads with index tid; the caller reduces.
 __device__ __forceinline__ float partial_square_sum(const ImmaParams& p, int m, int tid, int threads) {
-    const AnyRow row{static_cast<const uint8_t*>(p.x) + static_cast<size_t>(m) * p.k * (p.x_bf16 ? 2 : 4), p.x_bf16};
+    const AnyRow row = member_row(p, m);
     float acc = 0.0f;
+#pragma unroll 2
     for (int c = tid; c < p.k / 8; c += threads) {
         float v[8];
         load_row8(row + c * 8, v);
@@ -173,6 +214,13 @@ __device__ __forceinline__ float partial_square_sum(const ImmaParams& p, int m, 
         for (int j = 0; j < 8; ++j) acc = fmaf(v[j], v[j], acc);
     }
     return acc;
+}
+
+// D = A(16x32, s8, row) * B(32x8, s8, col), s32: the instruction of imma_zero with signed weights.
+__device__ __forceinline__ void imma_signed_zero(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+                 : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
 }
 
 // D = A(16x32, u8, row) * B(32x8, s8, col), s32.  Lane (g = lane / 4, t = lane % 4) holds
@@ -197,11 +245,14 @@ __device__ __forceinline__ void imma16_zero(int (&c)[4], uint32_t a0, uint32_t a
                  : "r"(a0), "r"(a1), "r"(b0), "r"(0));
 }
 
-// A 32-bit word of shared memory at `address`, which is two bytes past a word boundary when ODD.
-template <bool ODD>
+// A 32-bit word of shared memory at `address`: on a word boundary, two bytes past one, or one of the two by lane.
+enum Parity { kEven = 0, kOdd = 1, kMixed = 2 };
+template <int PARITY>
 __device__ __forceinline__ uint32_t lds32_shifted(uint32_t address) {
-    if (!ODD) return lds32(address);
-    return __funnelshift_r(lds32(address - 2), lds32(address + 2), 16);
+    if (PARITY == kEven) return lds32(address);
+    if (PARITY == kOdd) return __funnelshift_r(lds32(address - 2), lds32(address + 2), 16);
+    const uint32_t word = address & ~3u;
+    return __funnelshift_r(lds32(word), lds32(word + 4), (address & 3u) * 8u);
 }
 
 // Per-lane shared addresses at the super-block the warp works on.  Column g of column group q is plane g & 3 of
@@ -368,29 +419,29 @@ __device__ __forceinline__ void block_q6(uint32_t a0, uint32_t a1, const LaneX<G
 
 // The two blocks that share the ql word (N2, VLOW, H): block B = 8 N2 + 2 VLOW + H from its low nibbles, block B + 4 from
 // its high nibbles.
-template <int N2, int H, int VLOW, int GROUPS, bool ODD>
+template <int N2, int H, int VLOW, int GROUPS, int PARITY>
 __device__ __forceinline__ void blocks_q6(uint32_t p0, uint32_t p1, uint32_t qh0, uint32_t qh1, uint32_t lane_bytes, const LaneX<GROUPS>& lx,
                                           const uint32_t (&sc0)[4], const uint32_t (&sc1)[4], int (&total)[GROUPS][4]) {
     constexpr int B = 8 * N2 + 2 * VLOW + H;
-    const uint32_t ql0 = lds32_shifted<ODD>(p0 + 64 * N2 + 32 * VLOW + 16 * H + lane_bytes);
-    const uint32_t ql1 = lds32_shifted<ODD>(p1 + 64 * N2 + 32 * VLOW + 16 * H + lane_bytes);
+    const uint32_t ql0 = lds32_shifted<PARITY>(p0 + 64 * N2 + 32 * VLOW + 16 * H + lane_bytes);
+    const uint32_t ql1 = lds32_shifted<PARITY>(p1 + 64 * N2 + 32 * VLOW + 16 * H + lane_bytes);
     block_q6<B, GROUPS>(q6_signed_bytes<VLOW>(ql0, qh0), q6_signed_bytes<VLOW>(ql1, qh1), lx, sc0[B >> 2], sc1[B >> 2], total);
     block_q6<B + 4, GROUPS>(q6_signed_bytes<VLOW + 2>(ql0, qh0), q6_signed_bytes<VLOW + 2>(ql1, qh1), lx, sc0[(B + 4) >> 2], sc1[(B + 4) >> 2],
                             total);
 }
 
 // The four blocks that share the qh word (N2, H).
-template <int N2, int H, int GROUPS, bool ODD>
+template <int N2, int H, int GROUPS, int PARITY>
 __device__ __forceinline__ void quarter_q6(uint32_t p0, uint32_t p1, uint32_t lane_bytes, const LaneX<GROUPS>& lx, const uint32_t (&sc0)[4],
                                            const uint32_t (&sc1)[4], int (&total)[GROUPS][4]) {
-    const uint32_t qh0 = lds32_shifted<ODD>(p0 + 128 + 32 * N2 + 16 * H + lane_bytes);
-    const uint32_t qh1 = lds32_shifted<ODD>(p1 + 128 + 32 * N2 + 16 * H + lane_bytes);
-    blocks_q6<N2, H, 0, GROUPS, ODD>(p0, p1, qh0, qh1, lane_bytes, lx, sc0, sc1, total);
-    blocks_q6<N2, H, 1, GROUPS, ODD>(p0, p1, qh0, qh1, lane_bytes, lx, sc0, sc1, total);
+    const uint32_t qh0 = lds32_shifted<PARITY>(p0 + 128 + 32 * N2 + 16 * H + lane_bytes);
+    const uint32_t qh1 = lds32_shifted<PARITY>(p1 + 128 + 32 * N2 + 16 * H + lane_bytes);
+    blocks_q6<N2, H, 0, GROUPS, PARITY>(p0, p1, qh0, qh1, lane_bytes, lx, sc0, sc1, total);
+    blocks_q6<N2, H, 1, GROUPS, PARITY>(p0, p1, qh0, qh1, lane_bytes, lx, sc0, sc1, total);
 }
 
-// One Q6_K super-block of rows g (at p0) and g + 8 (at p1); ODD: the super-block starts two bytes past a word boundary.
-template <int GROUPS, bool ODD>
+// One Q6_K super-block of rows g (at p0) and g + 8 (at p1); PARITY: where they start with respect to a word.
+template <int GROUPS, int PARITY>
 __device__ __forceinline__ void superblock_q6(uint32_t p0, uint32_t p1, const LaneX<GROUPS>& lx, int t, float (&acc)[GROUPS][2]) {
     int total[GROUPS][4];
 #pragma unroll
@@ -402,13 +453,13 @@ __device__ __forceinline__ void superblock_q6(uint32_t p0, uint32_t p1, const La
     uint32_t sc0[4], sc1[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        sc0[i] = lds32_shifted<ODD>(p0 + 192 + 4 * i);
-        sc1[i] = lds32_shifted<ODD>(p1 + 192 + 4 * i);
+        sc0[i] = lds32_shifted<PARITY>(p0 + 192 + 4 * i);
+        sc1[i] = lds32_shifted<PARITY>(p1 + 192 + 4 * i);
     }
-    quarter_q6<0, 0, GROUPS, ODD>(p0, p1, lane_bytes, lx, sc0, sc1, total);
-    quarter_q6<0, 1, GROUPS, ODD>(p0, p1, lane_bytes, lx, sc0, sc1, total);
-    quarter_q6<1, 0, GROUPS, ODD>(p0, p1, lane_bytes, lx, sc0, sc1, total);
-    quarter_q6<1, 1, GROUPS, ODD>(p0, p1, lane_bytes, lx, sc0, sc1, total);
+    quarter_q6<0, 0, GROUPS, PARITY>(p0, p1, lane_bytes, lx, sc0, sc1, total);
+    quarter_q6<0, 1, GROUPS, PARITY>(p0, p1, lane_bytes, lx, sc0, sc1, total);
+    quarter_q6<1, 0, GROUPS, PARITY>(p0, p1, lane_bytes, lx, sc0, sc1, total);
+    quarter_q6<1, 1, GROUPS, PARITY>(p0, p1, lane_bytes, lx, sc0, sc1, total);
     const float d0 = f16_bits_to_f32(lds_u16(p0 + 208)), d1 = f16_bits_to_f32(lds_u16(p1 + 208));
     const float weight = (t & 1) ? 16384.0f : 1.0f;
 #pragma unroll
@@ -421,16 +472,98 @@ __device__ __forceinline__ void superblock_q6(uint32_t p0, uint32_t p1, const La
     }
 }
 
-// ---------------------------------------------------------------- the kernel
-// Shared-memory plan: [ring: stages x stage][zeros 1 KiB][image: planes | sums | scale][red: 2 x 8 warps x 128 f32]
-//                     [norm: 9 x 8 f32][barriers]
-__host__ __device__ inline size_t imma_fixed_bytes(int members, int nsb) {
-    return 128 /*alignment*/ + kZeroBytes + image_bytes(members, nsb) + 2 * kWarps * 128 * 4 + (kWarps + 1) * kMaxMembers * 4 + (2 * kMaxStages + 2) * 8;
+// ---- Q8_0: eight blocks of a 2-byte factor and 32 signed bytes stand for a super-block.  Blocks are 34 bytes, so in rows
+// that start on a word the quants of even blocks sit two bytes off a word and those of odd blocks on one.
+// An even block is taken as the words it does have: lane t takes words 1 + t and 5 + t behind the block's start; the last of
+// them, which lane 3 would share with the next block, is merged with the two quants behind the factor -- the K order
+// 2 .. 31, 0, 1 that the rotated image has for these blocks.
+// kRowsOdd: rows start anywhere; two words and a shift per operand word, image in plain order.
+template <int J, int GROUPS, bool ODD_ROWS>
+__device__ __forceinline__ void block_q8(uint32_t p0, uint32_t p1, const LaneX<GROUPS>& lx, int t, bool real, float (&sum)[GROUPS][2]) {
+    uint32_t a[2][2];
+    float d[2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const uint32_t block = (r == 0 ? p0 : p1) + 34 * J;
+        if constexpr (ODD_ROWS) {
+            const uint32_t start = block + 2 + 4 * static_cast<uint32_t>(t), word = start & ~3u, shift = (start & 3u) * 8u;
+            a[r][0] = __funnelshift_r(lds32(word), lds32(word + 4), shift);
+            a[r][1] = __funnelshift_r(lds32(word + 16), lds32(word + 20), shift);
+            d[r] = real ? f16_bits_to_f32(lds_u16(block)) : 0.0f;
+        } else if constexpr ((J & 1) == 0) {
+            const uint32_t first = lds32(block);   // factor, quants 0 and 1
+            a[r][0] = lds32(block + 4 + 4 * static_cast<uint32_t>(t));
+            const uint32_t last = lds32(block + 20 + 4 * static_cast<uint32_t>(t));
+            a[r][1] = t == 3 ? __byte_perm(last, first, 0x7610) : last;
+            d[r] = f16_bits_to_f32(first & 0xffffu);
+        } else {
+            a[r][0] = lds32(block + 2 + 4 * static_cast<uint32_t>(t));
+            a[r][1] = lds32(block + 18 + 4 * static_cast<uint32_t>(t));
+            d[r] = f16_bits_to_f32(lds_u16(block));
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < GROUPS; ++q) {
+        uint32_t b0, b1;
+        asm volatile("ld.shared.u32 %0, [%1+%2];" : "=r"(b0) : "r"(lx.x[q]), "n"(96 * J));
+        asm volatile("ld.shared.u32 %0, [%1+%2];" : "=r"(b1) : "r"(lx.x[q]), "n"(96 * J + 16));
+        int c[4];
+        imma_signed_zero(c, a[0][0], a[1][0], a[0][1], a[1][1], b0, b1);
+        // columns 2t, 2t + 1: planes p0 and p1 (t even, below 2^27 together), or p2 and zeros
+        sum[q][0] = fmaf(d[0], static_cast<float>(c[0] + 128 * c[1]), sum[q][0]);
+        sum[q][1] = fmaf(d[1], static_cast<float>(c[2] + 128 * c[3]), sum[q][1]);
+    }
 }
 
-template <uint32_t FMT, int GROUPS>
-__global__ void __launch_bounds__(kThreads, 2) gemv_imma_kernel(const __grid_constant__ CUtensorMap wmap, const ImmaParams p) {
-    using P = ImmaPlan<FMT>;
+// One group of eight Q8_0 blocks of rows g (at p0) and g + 8 (at p1); `blocks`: how many of them the row has.
+template <int GROUPS, bool ODD_ROWS>
+__device__ __forceinline__ void superblock_q8(uint32_t p0, uint32_t p1, const LaneX<GROUPS>& lx, int t, int blocks, float (&acc)[GROUPS][2]) {
+    float sum[GROUPS][2];
+#pragma unroll
+    for (int q = 0; q < GROUPS; ++q) sum[q][0] = sum[q][1] = 0.0f;
+    block_q8<0, GROUPS, ODD_ROWS>(p0, p1, lx, t, 0 < blocks, sum);
+    block_q8<1, GROUPS, ODD_ROWS>(p0, p1, lx, t, 1 < blocks, sum);
+    block_q8<2, GROUPS, ODD_ROWS>(p0, p1, lx, t, 2 < blocks, sum);
+    block_q8<3, GROUPS, ODD_ROWS>(p0, p1, lx, t, 3 < blocks, sum);
+    block_q8<4, GROUPS, ODD_ROWS>(p0, p1, lx, t, 4 < blocks, sum);
+    block_q8<5, GROUPS, ODD_ROWS>(p0, p1, lx, t, 5 < blocks, sum);
+    block_q8<6, GROUPS, ODD_ROWS>(p0, p1, lx, t, 6 < blocks, sum);
+    block_q8<7, GROUPS, ODD_ROWS>(p0, p1, lx, t, 7 < blocks, sum);
+    const float weight = (t & 1) ? 16384.0f : 1.0f;
+#pragma unroll
+    for (int q = 0; q < GROUPS; ++q) {
+        const float xs = __uint_as_float(lds32(lx.scale + 8 * q + 4 * (t >> 1))) * weight;
+        acc[q][0] = fmaf(xs, sum[q][0], acc[q][0]);
+        acc[q][1] = fmaf(xs, sum[q][1], acc[q][1]);
+    }
+}
+
+// ---------------------------------------------------------------- the kernel
+// Shared-memory plan: [ring: stages x stage][zeros 1 KiB][image: planes | sums | scale][red: groups x slots x 8 warps x 16 rows x
+//                     members of the column groups][norm: 2 x 9 x 8 f32][barriers]
+__host__ __device__ inline size_t imma_fixed_bytes(int members, int nsb, int slots) {
+    const size_t columns = static_cast<size_t>((members + 1) / 2 * 2);
+    return 128 /*alignment*/ + kZeroBytes + image_bytes(members, nsb) + kGroups * static_cast<size_t>(slots) * kGroupWarps * kTileRows * columns * 4 +
+           kGroups * kGroupWarps * kMaxMembers * 4 + (2 * kMaxStages + kGroups * kMaxSlots + 1) * 8;
+}
+
+// Where a CTA's stream of stages goes: chunk c (eight super-blocks) of its tiles, pairs of tiles interleaved chunk by chunk,
+// group g taking tile 2 i + g; an odd last tile is group 0's alone.
+struct Walk {
+    int stage, phase;
+    __device__ __forceinline__ void step(int items, int stages) {
+        stage += items;
+        if (stage >= stages) {
+            stage -= stages;
+            phase ^= 1;
+        }
+    }
+};
+
+template <uint32_t FMT, int FETCH, int GROUPS>
+__global__ void __launch_bounds__(kThreads, 1) gemv_imma_kernel(const __grid_constant__ CUtensorMap wmap, const ImmaParams p) {
+    using P = ImmaPlan<FMT, FETCH>;
+    constexpr int kColumns = 2 * GROUPS;   // members of the column groups
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((128u - (smem_addr(smem_raw) & 127u)) & 127u);
     uint8_t* ring = smem;
@@ -440,10 +573,11 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_imma_kernel(const __grid_con
     __half* sums = reinterpret_cast<__half*>(planes + image_plane_bytes(p.members, p.nsb));
     float* scale = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(sums) + image_sums_bytes(p.members, p.nsb));
     float* red = scale + static_cast<size_t>(p.nsb) * 8;
-    float* norm = red + 2 * kWarps * 128;
-    uint64_t* full = reinterpret_cast<uint64_t*>(norm + (kWarps + 1) * kMaxMembers);
+    float* norm = red + kGroups * p.slots * (kGroupWarps * kTileRows * kColumns);
+    uint64_t* full = reinterpret_cast<uint64_t*>(norm + kGroups * kGroupWarps * kMaxMembers);
     uint64_t* empty = full + kMaxStages;
-    uint64_t* image_bar = empty + kMaxStages;
+    uint64_t* summed = empty + kMaxStages;      // [group][slot]
+    uint64_t* image_bar = summed + kGroups * kMaxSlots;
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -451,154 +585,130 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_imma_kernel(const __grid_con
     pdl_launch_dependents();
     // The producer warp initialises the barriers and goes straight on to request weights; the consumers only
     // need to know that the barriers exist before their first wait (named barrier 2: they sync, the producer arrives).
-    if (warp == kWarps) {
-        if (lane == 0) {
-            tma_prefetch_descriptor(&wmap);
-            for (int s = 0; s < stages; ++s) {
-                mbar_init(&full[s], 1);
-                mbar_init(&empty[s], kWarps);
-            }
-            mbar_init(image_bar, 1);
-            mbar_fence_init();
+    if (warp == kConsumerWarps) {
+        if (lane == 0 && FETCH == kBoxes) tma_prefetch_descriptor(&wmap);
+        for (int b = lane; b < 2 * kMaxStages + kGroups * kMaxSlots + 1; b += 32) {
+            const bool is_empty = b >= kMaxStages && b < 2 * kMaxStages, is_summed = b >= 2 * kMaxStages && b < 2 * kMaxStages + kGroups * kMaxSlots;
+            mbar_init(&full[b], is_empty || is_summed ? kGroupWarps : 1);
         }
+        mbar_fence_init();
         __syncwarp();
         asm volatile("bar.arrive 2, %0;" ::"n"(kThreads) : "memory");
     }
 
-    const int tiles_total = (p.n + kTileRows - 1) / kTileRows;
-    const int tile_begin = static_cast<int>(static_cast<long long>(tiles_total) * blockIdx.x / gridDim.x);
-    const int tile_end = static_cast<int>(static_cast<long long>(tiles_total) * (blockIdx.x + 1) / gridDim.x);
-    const int tiles = tile_end - tile_begin;
-    const int chunks = (p.nsb + kWarps - 1) / kWarps;
-    const int total = tiles * chunks;
+    const int cta = static_cast<int>(blockIdx.x);
+    const int tile_begin = cta * p.tile_quotient + min(cta, p.tile_remainder);
+    const int tiles = p.tile_quotient + (cta < p.tile_remainder ? 1 : 0);
+    const int chunks = (p.nsb + kGroupWarps - 1) / kGroupWarps;
     bool ok = true;
 
-    if (warp == kWarps) {
+    if (warp == kConsumerWarps) {
         // ---------------- producer warp: the weight stream does not depend on the activations ----------------
-        if (lane == 0) {
-            bool image_requested = p.image == nullptr;
-            const int prefetch = min(total, stages);
-            auto request_image = [&]() {
-                // The image is the previous kernel's output; the first ring-full of weights is requested before it.
-                pdl_wait_prior();
-                const uint32_t bytes = static_cast<uint32_t>(image_bytes(p.members, p.nsb));
-                mbar_arrive_expect_tx(image_bar, bytes);
-                uint32_t done = 0;
-                while (done < bytes) {
-                    const uint32_t part = min(bytes - done, 32768u);
-                    bulk_copy_g2s(image + done, p.image + done, part, image_bar);
-                    done += part;
-                }
-                image_requested = true;
-            };
-            if (total == 0 && !image_requested) request_image();
-#pragma unroll 1
-            for (int it = 0; it < total; ++it) {
-                const int s = it % stages;
-                const int use = it / stages;
-                if (use > 0 && !mbar_wait_bounded_hint(&empty[s], (use - 1) & 1, 2000u)) {
-                    atomicExch(p.status, kDeviceWaitTimeout);
-                    break;
-                }
-                const int tile = it / chunks;
-                const int chunk = it - tile * chunks;
+        Walk walk{0, 1};   // the first round of every stage waits for nothing: parity 1 of a fresh barrier has passed
+        auto request = [&](int tile, int chunk) {
+            if (lane == 0 || FETCH != kBoxes) ok = ok && mbar_spin(&empty[walk.stage], walk.phase);
+            if (FETCH != kBoxes) ok = __all_sync(0xffffffffu, ok);
+            if (ok) {
                 const int row0 = (tile_begin + tile) * kTileRows;
-                const int sbs = min(kWarps, p.nsb - chunk * kWarps);
+                const int sbs = min(kGroupWarps, p.nsb - chunk * kGroupWarps);
                 const int boxes = (sbs + P::kBoxSb - 1) / P::kBoxSb;
-                mbar_arrive_expect_tx(&full[s], static_cast<uint32_t>(boxes * P::kBoxBytes));
-                for (int b = 0; b < boxes; ++b)
-                    tma_load_2d(ring + static_cast<size_t>(s) * P::kStageBytes + b * P::kBoxBytes, &wmap,
-                                (chunk * kWarps + b * P::kBoxSb) * P::kSbBytes / 8, row0, &full[s]);
-                if (it == prefetch - 1 && !image_requested) request_image();
+                uint8_t* stage = ring + static_cast<size_t>(walk.stage) * P::kStageBytes;
+                uint64_t* bar = &full[walk.stage];
+                if constexpr (FETCH == kBoxes) {
+                    if (lane == 0) {
+                        mbar_arrive_expect_tx(bar, static_cast<uint32_t>(boxes * P::kBoxBytes));
+                        const int x = chunk * (P::kBoxesPerStage * P::kBoxSpan / 8);
+                        for (int b = 0; b < boxes; ++b) tma_load_2d(stage + b * P::kBoxBytes, &wmap, x + b * (P::kBoxSpan / 8), row0, bar);
+                    }
+                } else {
+                    // lane = (box, row): the row's share of the box from the 16-byte boundary below, up to the one above
+                    static_assert(P::kBoxesPerStage * kTileRows <= 32, "one copy per lane");
+                    const int row = lane & (kTileRows - 1), b = lane >> 4;
+                    const unsigned long long row_start = static_cast<unsigned long long>(row0 + row) * p.row_bytes;
+                    const unsigned long long from = row_start + static_cast<unsigned long long>(chunk * P::kBoxesPerStage + b) * P::kBoxSpan;
+                    const unsigned long long to = min(from + P::kBoxSpan, row_start + p.row_bytes);
+                    const unsigned long long first = from & ~15ull;
+                    const bool mine = b < boxes && row0 + row < p.n;
+                    const uint32_t bytes = mine ? static_cast<uint32_t>(((to + 15ull) & ~15ull) - first) : 0u;
+                    const uint32_t total = __reduce_add_sync(0xffffffffu, bytes);
+                    if (lane == 0) mbar_arrive_expect_tx(bar, total);
+                    __syncwarp();
+                    if (mine) bulk_copy_g2s(stage + b * P::kBoxBytes + row * P::kRowPitch, p.weights + first, bytes, bar);
+                }
+            }
+            walk.step(1, stages);
+        };
+#pragma unroll 1
+        for (int tile = 0; tile < tiles; tile += 2) {
+            const int both = tile + 1 < tiles ? 2 : 1;
+#pragma unroll 1
+            for (int chunk = 0; chunk < chunks; ++chunk) {
+                request(tile, chunk);
+                if (both == 2) request(tile + 1, chunk);
             }
         }
+        ok = __all_sync(0xffffffffu, ok);
     } else {
         // ---------------- consumers ----------------
+        const int group = warp / kGroupWarps, w8 = warp % kGroupWarps;
         const int g = lane >> 2, t = lane & 3;
+        if (threadIdx.x < kZeroBytes / 4) reinterpret_cast<uint32_t*>(zeros)[threadIdx.x] = 0u;
         named_barrier_sync(2, kThreads);
-        // 256 consumers x 4 bytes = the zero area, in place (and visible to every warp) before the wait for the previous
-        // kernel ends: after that wait a warp only needs what it converts itself
-        reinterpret_cast<uint32_t*>(zeros)[threadIdx.x] = 0u;
-        named_barrier_sync(1, kConsumers);
         pdl_wait_prior();   // the activations may be the previous kernel's output, and y may still be read by it
-        const int owned_slices = p.nsb > warp ? (p.nsb - warp + kWarps - 1) / kWarps : 0;
-        if (p.image == nullptr && p.mode == 1 && p.members == 1 && p.nsb <= 2 * kWarps) {
-            // One row of at most sixteen super-blocks to normalise (a decode step's projections): every lane keeps its
-            // share of the warp's one or two slices in registers, so the row and the norm weights are read once -- one
-            // round trip to memory instead of three.  Sums run in the order of the general path below (same bits).
-            const AnyRow row{static_cast<const uint8_t*>(p.x), p.x_bf16};
-            float v[2][8], gain[2][8];
-            float part = 0.0f;
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                if (i < owned_slices) {
-                    const int k0 = (warp + i * kWarps) * kSuperBlock + lane * 8;
-                    load_row8(row + k0, v[i]);
-                    load_x8<float>(p.norm_weight + k0, gain[i]);
-                }
+        if (p.image != nullptr) {
+            // a consumer asks for the image: the producer may be far behind the previous kernel's end, filling the ring
+            if (threadIdx.x == 0) {
+                const uint32_t bytes = static_cast<uint32_t>(image_bytes(p.members, p.nsb));
+                mbar_arrive_expect_tx(image_bar, bytes);
+                for (uint32_t done = 0; done < bytes; done += 32768u) bulk_copy_g2s(image + done, p.image + done, min(bytes - done, 32768u), image_bar);
             }
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-                if (i < owned_slices)
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) part = fmaf(v[i][j], v[i][j], part);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-            if (lane == 0) norm[warp * kMaxMembers] = part;
-            named_barrier_sync(1, kConsumers);
-            float totalsq = 0.0f;
-#pragma unroll
-            for (int w = 0; w < kWarps; ++w) totalsq += norm[w * kMaxMembers];
-            const float inv_rms = 1.0f / sqrtf(totalsq / static_cast<float>(p.k) + p.eps);
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                if (i < owned_slices) {
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) v[i][j] = v[i][j] * inv_rms * gain[i][j];
-                    store_slice(0, warp + i * kWarps, lane, v[i], planes, sums, scale);
-                }
-            }
-            __syncwarp();   // a warp reads only the super-blocks it converted itself
-        } else if (p.image == nullptr) {
-            // norm[64 + m] = 1 / rms of member row m when RMSNorm is asked for
-            if (p.mode == 1) {
-                for (int m = 0; m < p.members; ++m) {
-                    float part = partial_square_sum(p, m, static_cast<int>(threadIdx.x), kConsumers);
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-                    if (lane == 0) norm[warp * kMaxMembers + m] = part;
-                }
-                named_barrier_sync(1, kConsumers);
-                if (threadIdx.x < kMaxMembers) {
-                    float totalsq = 0.0f;
-#pragma unroll
-                    for (int w = 0; w < kWarps; ++w) totalsq += norm[w * kMaxMembers + threadIdx.x];
-                    norm[kWarps * kMaxMembers + threadIdx.x] = 1.0f / sqrtf(totalsq / static_cast<float>(p.k) + p.eps);
-                }
-                named_barrier_sync(1, kConsumers);
-            }
-            // The warp's slices (super-blocks warp, warp + 8, ... of every member), two loads in flight.
-            const float* inv_rms = norm + kWarps * kMaxMembers;
-            const int slices = owned_slices * p.members;
+        } else {
+            // The warp's slices (every sixteenth of [member][super-block]); the next one is on its way while one is converted.  One
+            // copy of the code: it runs once or twice, and most of its time is fetching the instructions.
+            float* my_norm = norm + group * kGroupWarps * kMaxMembers;   // both groups make the same sums
+            float v[8], by[8];
+            int m = 0, sb = warp, held_m = 0, held_sb = -1;
 #pragma unroll 1
-            for (int i = 0; i < slices; i += 2) {
-                const int sb0 = warp + (i / p.members) * kWarps, m0 = i % p.members;
-                const bool second = i + 1 < slices;
-                const int i1 = second ? i + 1 : i;
-                const int sb1 = warp + (i1 / p.members) * kWarps, m1 = i1 % p.members;
-                float v0[8], v1[8];
-                load_slice(p, m0, sb0, lane, p.mode == 1 ? inv_rms[m0] : 1.0f, v0);
-                load_slice(p, m1, sb1, lane, p.mode == 1 ? inv_rms[m1] : 1.0f, v1);
-                store_slice(m0, sb0, lane, v0, planes + static_cast<size_t>(m0) * p.nsb * kSliceBytes, sums + static_cast<size_t>(m0) * p.nsb * 16, scale);
-                if (second)
-                    store_slice(m1, sb1, lane, v1, planes + static_cast<size_t>(m1) * p.nsb * kSliceBytes, sums + static_cast<size_t>(m1) * p.nsb * 16,
-                                scale);
+            for (;;) {
+                while (sb >= p.nsb && m < p.members) {
+                    sb -= p.nsb;
+                    ++m;
+                }
+                float next[8], next_by[8];
+                if (m < p.members) load_slice(p, m, sb, lane, next, next_by);
+                if (held_sb >= 0) {
+                    float inv_rms = 1.0f;
+                    if (p.mode == 1) {
+                        float totalsq = 0.0f;
+#pragma unroll
+                        for (int w = 0; w < kGroupWarps; ++w) totalsq += my_norm[w * kMaxMembers + held_m];
+                        inv_rms = 1.0f / sqrtf(totalsq / static_cast<float>(p.k) + p.eps);
+                    }
+                    apply_prologue(p, inv_rms, v, by);
+                    store_slice(p.rotated != 0, held_m, held_sb, lane, v, planes + static_cast<size_t>(held_m) * p.nsb * kSliceBytes,
+                                sums + static_cast<size_t>(held_m) * p.nsb * 16, scale);
+                } else if (p.mode == 1) {
+                    for (int row = 0; row < p.members; ++row) {
+                        float part = partial_square_sum(p, row, w8 * 32 + lane, kGroupWarps * 32);
+#pragma unroll
+                        for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+                        if (lane == 0) my_norm[w8 * kMaxMembers + row] = part;
+                    }
+                    named_barrier_sync(3 + group, kGroupWarps * 32);
+                }
+                if (m >= p.members) break;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    v[j] = next[j];
+                    by[j] = next_by[j];
+                }
+                held_m = m;
+                held_sb = sb;
+                sb += kConsumerWarps;
             }
-            __syncwarp();   // a warp reads only the super-blocks it converted itself
-        } else if (!mbar_wait_bounded(image_bar, 0)) {
-            atomicExch(p.status, kDeviceWaitTimeout);
-            ok = false;
         }
+        named_barrier_sync(1, kConsumers);   // the zero area, and the slices the other warps converted
+        if (p.image != nullptr) ok = mbar_spin(image_bar, 0);
 
         LaneX<GROUPS> lx;
         {
@@ -606,8 +716,8 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_imma_kernel(const __grid_con
             for (int q = 0; q < GROUPS; ++q) {
                 const int member = 2 * q + (g >> 2), plane = g & 3;
                 const bool real = member < p.members && plane < 3;
-                // the lane's share of a block: 8 bytes of a 32-weight sub-block (Q4_K / Q5_K), 4 bytes of a 16-weight block (Q6_K)
-                const uint32_t lane_bytes = (FMT == kQ6_K ? 4u : 8u) * t;
+                // the lane's share of a block: 8 bytes of a 32-weight sub-block (Q4_K / Q5_K), 4 bytes of 16 weights (Q6_K, Q8_0)
+                const uint32_t lane_bytes = (FMT == kQ6_K || FMT == kQ8_0 ? 4u : 8u) * t;
                 lx.x[q] = real ? smem_addr(planes) + static_cast<uint32_t>(member) * static_cast<uint32_t>(p.nsb) * kSliceBytes + plane * 32u + lane_bytes
                                : smem_addr(zeros) + 96u + lane_bytes;
                 lx.step[q] = real ? static_cast<uint32_t>(kSliceBytes) : 0u;
@@ -615,85 +725,113 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_imma_kernel(const __grid_con
             const uint32_t sums_member = g < p.members ? static_cast<uint32_t>(g) : 0u;
             lx.sums = smem_addr(sums) + sums_member * static_cast<uint32_t>(p.nsb) * 32u;
             lx.scale = smem_addr(scale);
-            lx.advance(warp);   // the warp's super-block of the first chunk
         }
-        const uint32_t ring_addr = smem_addr(ring);
-        // This warp's super-block inside a stage: box warp / kBoxSb, position warp % kBoxSb, rows g and g + 8.
-        const uint32_t lane_off = static_cast<uint32_t>((warp / P::kBoxSb) * P::kBoxBytes + (warp % P::kBoxSb) * P::kSbBytes + g * P::kRowPitch);
+        // This warp's super-block inside a stage: box w8 / kBoxSb, position w8 % kBoxSb, rows g and g + 8.
+        const uint32_t ring_addr = smem_addr(ring) + static_cast<uint32_t>((w8 / P::kBoxSb) * P::kBoxBytes + (w8 % P::kBoxSb) * P::kSbBytes + g * P::kRowPitch);
+        lx.advance(w8);   // the warp's super-block of the first chunk
+        Walk walk{0, 0};
+        walk.step(tiles > 1 ? group : 0, stages);
+        int slot = 0, slot_phase = 0, turn = 0;   // of the group's next tile: where its sums meet, and which warp finishes it
 
 #pragma unroll 1
-        for (int tile = 0; tile < tiles; ++tile) {
+        for (int tile = group; tile < tiles; tile += kGroups) {
+            const int row0 = (tile_begin + tile) * kTileRows;
             float acc[GROUPS][2], mins[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
             for (int q = 0; q < GROUPS; ++q) acc[q][0] = acc[q][1] = 0.0f;
+            const int items = (tile | 1) < tiles ? kGroups : 1;   // stages from one chunk of this tile to its next
+            uint32_t delta0 = 0u, delta1 = 0u;   // how far behind the copied boundary the rows start
+            if (FETCH != kBoxes) {
+                delta0 = static_cast<uint32_t>(static_cast<unsigned long long>(row0 + g) * p.row_bytes) & 15u;
+                delta1 = (delta0 + 8u * static_cast<uint32_t>(p.row_bytes)) & 15u;
+            }
 #pragma unroll 1
             for (int chunk = 0; chunk < chunks; ++chunk) {
-                const int it = tile * chunks + chunk;
-                const int s = it % stages;
-                if (ok && !mbar_wait_bounded_hint(&full[s], (it / stages) & 1, 2000u)) {
-                    atomicExch(p.status, kDeviceWaitTimeout);
-                    ok = false;
-                }
-                const int sb = chunk * kWarps + warp;
+                ok = ok && mbar_spin(&full[walk.stage], walk.phase);
+                const int sb = chunk * kGroupWarps + w8;
                 if (sb < p.nsb) {
-                    const uint32_t p0 = ring_addr + static_cast<uint32_t>(s) * P::kStageBytes + lane_off;
+                    const uint32_t base = ring_addr + static_cast<uint32_t>(walk.stage) * P::kStageBytes;
+                    const uint32_t p0 = base + delta0, p1 = base + 8 * P::kRowPitch + delta1;
                     if constexpr (FMT == kQ6_K) {
-                        // 210-byte super-blocks: the warp's one starts on a word boundary when its position in the box is even
-                        if (warp & 1) superblock_q6<GROUPS, true>(p0, p0 + 8 * P::kRowPitch, lx, t, acc);
-                        else superblock_q6<GROUPS, false>(p0, p0 + 8 * P::kRowPitch, lx, t, acc);
+                        // 210-byte super-blocks: in rows that start on a word the warp's one does when its position in the box is even
+                        if constexpr (FETCH == kRowsOdd) superblock_q6<GROUPS, kMixed>(p0, p1, lx, t, acc);
+                        else if (w8 & 1) superblock_q6<GROUPS, kOdd>(p0, p1, lx, t, acc);
+                        else superblock_q6<GROUPS, kEven>(p0, p1, lx, t, acc);
+                    } else if constexpr (FMT == kQ8_0) {
+                        superblock_q8<GROUPS, FETCH != kBoxes>(p0, p1, lx, t, p.k / 32 - sb * 8, acc);
                     } else {
-                        superblock<FMT, GROUPS>(p0, p0 + 8 * P::kRowPitch, lx, t, acc, mins);
+                        superblock<FMT, GROUPS>(p0, p1, lx, t, acc, mins);
                     }
                 }
-                lx.advance(kWarps);
+                lx.advance(kGroupWarps);
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&empty[s]);
+                if (lane == 0) mbar_arrive(&empty[walk.stage]);
+                // behind the tile's last chunk: the first of the group's next tile is one full pair's stride on
+                walk.step(items, stages);
             }
-            lx.advance(-chunks * kWarps);
-            // Tile end: a member's two plane shares sit in neighbouring lanes; then the eight warps' partial sums
-            // (each 16 rows x 8 members) meet in shared memory, the minima terms added by the lanes that hold them.
-            float* buf = red + (tile & 1) * (kWarps * 128) + warp * 128;
+            lx.advance(-chunks * kGroupWarps);
+            // Tile end: a member's two plane shares sit in neighbouring lanes and its minima in lane q of the four; the eight warps'
+            // partial sums meet in a slot of shared memory, and one warp -- each in turn -- adds them and stores the rows.  The
+            // others go on: a slot is written again only by a warp that has seen a stage which the finisher gave back later.
+            float* part = red + (group * p.slots + slot) * (kGroupWarps * kTileRows * kColumns);
+            float* buf = part + w8 * (kTileRows * kColumns);
 #pragma unroll
             for (int q = 0; q < GROUPS; ++q) {
-                const float v0 = acc[q][0] + __shfl_xor_sync(0xffffffffu, acc[q][0], 1);
-                const float v1 = acc[q][1] + __shfl_xor_sync(0xffffffffu, acc[q][1], 1);
+                float v0 = acc[q][0] + __shfl_xor_sync(0xffffffffu, acc[q][0], 1);
+                float v1 = acc[q][1] + __shfl_xor_sync(0xffffffffu, acc[q][1], 1);
+                if (FMT == kQ4_K || FMT == kQ5_K) {
+                    const int holder = (lane & ~3) | q;
+                    const float m0 = __shfl_sync(0xffffffffu, mins[0], holder), m1 = __shfl_sync(0xffffffffu, mins[1], holder);
+                    const float m2 = __shfl_sync(0xffffffffu, mins[2], holder), m3 = __shfl_sync(0xffffffffu, mins[3], holder);
+                    v0 += t < 2 ? m0 : m1;
+                    v1 += t < 2 ? m2 : m3;
+                }
                 if ((t & 1) == 0) {
-                    buf[g * 8 + 2 * q + (t >> 1)] = v0;
-                    buf[(g + 8) * 8 + 2 * q + (t >> 1)] = v1;
+                    buf[g * kColumns + 2 * q + (t >> 1)] = v0;
+                    buf[(g + 8) * kColumns + 2 * q + (t >> 1)] = v1;
                 }
             }
             __syncwarp();
-            if (2 * t < 2 * GROUPS) {
-                buf[g * 8 + 2 * t] += mins[0];
-                buf[g * 8 + 2 * t + 1] += mins[1];
-                buf[(g + 8) * 8 + 2 * t] += mins[2];
-                buf[(g + 8) * 8 + 2 * t + 1] += mins[3];
-            }
-            named_barrier_sync(1, kConsumers);
-            if (threadIdx.x < 128) {
-                const int row = static_cast<int>(threadIdx.x) >> 3, m = static_cast<int>(threadIdx.x) & 7;
-                const long long out_row = static_cast<long long>(tile_begin + tile) * kTileRows + row;
-                if (m < p.members && out_row < p.n) {
-                    const float* all = red + (tile & 1) * (kWarps * 128);
-                    float v = all[threadIdx.x];
+            uint64_t* bar = &summed[group * kMaxSlots + slot];
+            if (lane == 0) mbar_arrive(bar);
+            if (w8 == turn) {
+                constexpr int kOutputs = kTileRows * kColumns / 32;   // per lane
+                float old[kOutputs];
 #pragma unroll
-                    for (int w = 1; w < kWarps; ++w) v += all[w * 128 + threadIdx.x];
-                    const size_t o = static_cast<size_t>(m) * p.n + static_cast<size_t>(out_row);
-                    if (p.y_bf16) {
-                        if (p.accumulate) v += __bfloat162float(static_cast<const __nv_bfloat16*>(p.y)[o]);
-                        static_cast<__nv_bfloat16*>(p.y)[o] = __float2bfloat16_rn(v);
-                    } else {
-                        if (p.accumulate) v += static_cast<const float*>(p.y)[o];
-                        static_cast<float*>(p.y)[o] = v;
+                for (int i = 0; i < kOutputs; ++i) {
+                    const int item = i * 32 + lane, m = item % kColumns, row = row0 + item / kColumns;
+                    old[i] = 0.0f;
+                    if (p.accumulate && m < p.members && row < p.n) {
+                        const size_t o = static_cast<size_t>(m) * p.n + static_cast<size_t>(row);
+                        old[i] = p.y_bf16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(p.y)[o]) : static_cast<const float*>(p.y)[o];
+                    }
+                }
+                ok = ok && mbar_spin(bar, slot_phase);
+#pragma unroll
+                for (int i = 0; i < kOutputs; ++i) {
+                    const int item = i * 32 + lane, m = item % kColumns, row = row0 + item / kColumns;
+                    float v = part[item];
+#pragma unroll
+                    for (int w = 1; w < kGroupWarps; ++w) v += part[w * (kTileRows * kColumns) + item];
+                    if (m < p.members && row < p.n) {
+                        const size_t o = static_cast<size_t>(m) * p.n + static_cast<size_t>(row);
+                        if (p.accumulate) v += old[i];
+                        if (p.y_bf16) static_cast<__nv_bfloat16*>(p.y)[o] = __float2bfloat16_rn(v);
+                        else static_cast<float*>(p.y)[o] = v;
                     }
                 }
             }
+            turn = (turn + 1) % kGroupWarps;
+            if (++slot == p.slots) {
+                slot = 0;
+                slot_phase ^= 1;
+            }
         }
     }
-    // Common exit: after a wait that ran out, copies may still be in flight into this CTA's shared memory;
-    // give them time to land before the memory is handed to another CTA.
-    __syncthreads();
-    if (*reinterpret_cast<volatile int*>(p.status) != kDeviceOk) {
+    // A wait that ran out: copies may still be in flight into this CTA's shared memory; give them time to land before the
+    // memory is handed to another CTA.  (Otherwise every copy has been waited for by the consumers.)
+    if (!ok) {
+        atomicExch(p.status, kDeviceWaitTimeout);
         for (int spin = 0; spin < 64; ++spin) __nanosleep(1000);
     }
 }
@@ -722,30 +860,82 @@ __global__ void __launch_bounds__(256) gemv_imma_image_kernel(const ImmaParams p
     float* scale = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(sums) + image_sums_bytes(p.members, p.nsb));
     const int sb = blockIdx.x * 8 + warp;
     if (sb < p.nsb) {
-        float v[8];
-        load_slice(p, m, sb, lane, inv_rms, v);
-        store_slice(m, sb, lane, v, image + static_cast<size_t>(m) * p.nsb * kSliceBytes, sums + static_cast<size_t>(m) * p.nsb * 16, scale);
+        float v[8], by[8];
+        load_slice(p, m, sb, lane, v, by);
+        apply_prologue(p, inv_rms, v, by);
+        store_slice(p.rotated != 0, m, sb, lane, v, image + static_cast<size_t>(m) * p.nsb * kSliceBytes, sums + static_cast<size_t>(m) * p.nsb * 16, scale);
     }
 }
 
 constexpr size_t kSmemLimit = 227 * 1024;
 
-template <uint32_t FMT, int GROUPS>
+int block_bytes(uint32_t value_type) { return value_type == kQ8_0 ? 34 : value_type == kQ4_K ? 144 : value_type == kQ5_K ? 176 : 210; }
+int superblocks(int k) { return (k + kSuperBlock - 1) / kSuperBlock; }
+unsigned long long encoded_row_bytes(uint32_t value_type, int k) {
+    return value_type == kQ8_0 ? static_cast<unsigned long long>(k / 32) * 34 : static_cast<unsigned long long>(k / kSuperBlock) * block_bytes(value_type);
+}
+Fetch fetch_of(uint32_t value_type, int k) {
+    const unsigned long long row = encoded_row_bytes(value_type, k);
+    if (row % 16 == 0) return kBoxes;
+    return row % 4 == 0 && value_type == kQ6_K ? kRowsEven : kRowsOdd;
+}
+
+// Stages and slots of a launch; stages = 0 when fewer than two fit.
+struct Ring {
+    int stages, slots;
+};
+Ring ring_of(size_t stage_bytes, int members, int nsb, int items, int wanted) {
+    const int chunks = (nsb + kGroupWarps - 1) / kGroupWarps;
+    for (int stages = kMaxStages; stages >= 2; --stages) {
+        if (wanted > 0 && stages > wanted && stages > 2) continue;
+        if (stages > 2 && stages > items) continue;   // no more than the CTA has use for
+        // A warp that writes the slot of the group's tile T + slots has seen its last stage, and every warp of the group has given
+        // back all stages of the ring's length earlier; the first stage of tile T + 1 must be among them.
+        const int slots = 1 + (stages + 1 > chunks ? (stages + 1 - chunks + 2 * chunks - 1) / (2 * chunks) : 0);
+        if (imma_fixed_bytes(members, nsb, slots) + stages * stage_bytes <= kSmemLimit) return Ring{stages, slots};
+    }
+    return Ring{0, 0};
+}
+size_t stage_bytes_of(uint32_t value_type, Fetch fetch) {
+    switch (value_type) {
+        case kQ4_K: return ImmaPlan<kQ4_K, kBoxes>::kStageBytes;
+        case kQ5_K: return ImmaPlan<kQ5_K, kBoxes>::kStageBytes;
+        case kQ6_K: return fetch == kBoxes ? ImmaPlan<kQ6_K, kBoxes>::kStageBytes : ImmaPlan<kQ6_K, kRowsEven>::kStageBytes;
+        default: return ImmaPlan<kQ8_0, kBoxes>::kStageBytes;
+    }
+}
+
+ImmaParams params_of(const MmaGemvArgs& a) {
+    ImmaParams p{};
+    p.x = a.x;
+    p.x_bf16 = a.x_bf16 ? 1 : 0;
+    p.mode = a.mode;
+    p.norm_weight = a.norm_weight;
+    p.eps = a.eps;
+    p.rotated = gemv_imma_rotates(a.value_type, a.k) ? 1 : 0;
+    p.k = a.k;
+    p.nsb = superblocks(a.k);
+    p.members = a.members;
+    return p;
+}
+
+template <uint32_t FMT, int FETCH, int GROUPS>
 cudaError_t launch_groups(const MmaGemvArgs& a) {
-    using P = ImmaPlan<FMT>;
-    auto kernel = gemv_imma_kernel<FMT, GROUPS>;
-    const int nsb = a.k / kSuperBlock;
-    const size_t fixed = imma_fixed_bytes(a.members, nsb);
-    // Two CTAs per SM when each then has at least two stages, else one.
-    auto share = [](int ctas) { return (kSmemLimit - 1024 * static_cast<size_t>(ctas)) / static_cast<size_t>(ctas); };
-    int resident = fixed + 2 * static_cast<size_t>(P::kStageBytes) <= share(2) ? 2 : 1;
-    if (a.resident > 0 && a.resident < resident) resident = a.resident;
-    const size_t budget = share(resident);
-    int stages = static_cast<int>((budget - fixed) / P::kStageBytes);
-    if (stages > kMaxStages) stages = kMaxStages;
-    if (a.stages > 0 && a.stages < stages) stages = a.stages;
-    if (stages < 2) return cudaErrorInvalidConfiguration;
-    const size_t smem = fixed + static_cast<size_t>(stages) * P::kStageBytes;
+    using P = ImmaPlan<FMT, FETCH>;
+    auto kernel = gemv_imma_kernel<FMT, FETCH, GROUPS>;
+    ImmaParams p = params_of(a);
+    // One CTA per SM: its sixteen consumer warps share one image of the activations, and whole SMs divide the tiles more
+    // evenly than halves do.
+    const int tiles = (a.n + kTileRows - 1) / kTileRows, chunks = (p.nsb + kGroupWarps - 1) / kGroupWarps;
+    const int grid = tiles < a.sm_count ? tiles : a.sm_count;
+    p.tile_quotient = tiles / grid;
+    p.tile_remainder = tiles % grid;
+    const int items = (p.tile_quotient + (p.tile_remainder > 0 ? 1 : 0)) * chunks;
+    const Ring ring = ring_of(P::kStageBytes, a.members, p.nsb, items, a.stages);
+    if (ring.stages == 0) return cudaErrorInvalidConfiguration;
+    p.stages = ring.stages;
+    p.slots = ring.slots;
+    const size_t smem = imma_fixed_bytes(a.members, p.nsb, p.slots) + static_cast<size_t>(p.stages) * P::kStageBytes;
     static int configured_device = -1;
     int device = 0;
     cudaGetDevice(&device);
@@ -754,84 +944,67 @@ cudaError_t launch_groups(const MmaGemvArgs& a) {
         if (e != cudaSuccess) return e;
         configured_device = device;
     }
-    EncodeTiledFn encode = encode_tiled_fn();
-    if (encode == nullptr) return cudaErrorNotSupported;
-    const unsigned long long row_bytes = static_cast<unsigned long long>(nsb) * P::kSbBytes;
-    CUtensorMap wmap;
-    const cuuint64_t dims[2] = {static_cast<cuuint64_t>(row_bytes / 8), static_cast<cuuint64_t>(a.n)};
-    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(row_bytes)};
-    const cuuint32_t box[2] = {static_cast<cuuint32_t>(P::kRowPitch / 8), static_cast<cuuint32_t>(kTileRows)};
-    const cuuint32_t elem[2] = {1, 1};
-    if (encode(&wmap, CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, const_cast<uint8_t*>(a.weights), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return cudaErrorInvalidValue;
-    ImmaParams p{};
-    p.x = a.x;
-    p.x_bf16 = a.x_bf16 ? 1 : 0;
-    p.mode = a.mode;
-    p.norm_weight = a.norm_weight;
-    p.eps = a.eps;
+    p.row_bytes = encoded_row_bytes(FMT, a.k);
+    CUtensorMap wmap{};
+    if constexpr (FETCH == kBoxes) {
+        EncodeTiledFn encode = encode_tiled_fn();
+        if (encode == nullptr) return cudaErrorNotSupported;
+        const cuuint64_t dims[2] = {static_cast<cuuint64_t>(p.row_bytes / 8), static_cast<cuuint64_t>(a.n)};
+        const cuuint64_t strides[1] = {static_cast<cuuint64_t>(p.row_bytes)};
+        const cuuint32_t box[2] = {static_cast<cuuint32_t>(P::kRowPitch / 8), static_cast<cuuint32_t>(kTileRows)};
+        const cuuint32_t elem[2] = {1, 1};
+        if (encode(&wmap, CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, const_cast<uint8_t*>(a.weights), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return cudaErrorInvalidValue;
+    }
     p.image = static_cast<const uint8_t*>(a.image);
+    p.weights = a.weights;
     p.y = a.y;
     p.y_bf16 = a.y_bf16 ? 1 : 0;
     p.accumulate = a.accumulate ? 1 : 0;
-    p.k = a.k;
     p.n = a.n;
-    p.nsb = nsb;
-    p.members = a.members;
-    p.stages = stages;
     p.status = a.device_status;
-    const int tiles = (a.n + kTileRows - 1) / kTileRows;
-    int per_sm = resident;
-    if (a.grid_ctas > 0) per_sm = a.grid_ctas < resident ? a.grid_ctas : resident;
-    int grid = a.sm_count * per_sm;
-    if (grid > tiles) grid = tiles;
     return launch_kernel(kernel, dim3(grid), dim3(kThreads), smem, a.stream, wmap, p);
 }
 
-template <uint32_t FMT>
+template <uint32_t FMT, int FETCH>
 cudaError_t launch_format(const MmaGemvArgs& a) {
     switch ((a.members + 1) / 2) {
-        case 1: return launch_groups<FMT, 1>(a);
-        case 2: return launch_groups<FMT, 2>(a);
-        case 3: return launch_groups<FMT, 3>(a);
-        default: return launch_groups<FMT, 4>(a);
+        case 1: return launch_groups<FMT, FETCH, 1>(a);
+        case 2: return launch_groups<FMT, FETCH, 2>(a);
+        case 3: return launch_groups<FMT, FETCH, 3>(a);
+        default: return launch_groups<FMT, FETCH, 4>(a);
     }
 }
 
 }  // namespace
 
+bool gemv_imma_rotates(uint32_t value_type, int k) { return value_type == kQ8_0 && fetch_of(value_type, k) == kBoxes; }
+
 bool gemv_imma_supports(uint32_t value_type, int k, int n, int members, const void* weights) {
-    if (value_type != kQ4_K && value_type != kQ5_K && value_type != kQ6_K) return false;
-    if (members < 1 || members > kMaxMembers || k <= 0 || k % kSuperBlock != 0 || n < kTileRows) return false;
-    const int block_bytes = value_type == kQ4_K ? 144 : value_type == kQ5_K ? 176 : 210;
-    const unsigned long long row_bytes = static_cast<unsigned long long>(k / kSuperBlock) * block_bytes;
-    if (row_bytes % 16 != 0 || reinterpret_cast<uintptr_t>(weights) % 16 != 0) return false;   // Q6_K: K / 256 a multiple of eight
-    const size_t stage = value_type == kQ4_K ? ImmaPlan<kQ4_K>::kStageBytes : value_type == kQ5_K ? ImmaPlan<kQ5_K>::kStageBytes
-                                                                                                  : ImmaPlan<kQ6_K>::kStageBytes;
-    return imma_fixed_bytes(members, k / kSuperBlock) + 2 * stage <= kSmemLimit - 1024;
+    if (value_type != kQ4_K && value_type != kQ5_K && value_type != kQ6_K && value_type != kQ8_0) return false;
+    if (members < 1 || members > kMaxMembers || k <= 0 || k % (value_type == kQ8_0 ? 32 : kSuperBlock) != 0 || n < kTileRows) return false;
+    if (reinterpret_cast<uintptr_t>(weights) % 16 != 0) return false;
+    return ring_of(stage_bytes_of(value_type, fetch_of(value_type, k)), members, superblocks(k), 2, 0).stages != 0;
 }
 
-size_t gemv_imma_image_bytes(int members, int k) { return (image_bytes(members, k / kSuperBlock) + 255) & ~static_cast<size_t>(255); }
+size_t gemv_imma_image_bytes(int members, int k) { return (image_bytes(members, superblocks(k)) + 255) & ~static_cast<size_t>(255); }
 
 cudaError_t launch_gemv_imma_image(const MmaGemvArgs& a, void* image) {
-    ImmaParams p{};
-    p.x = a.x;
-    p.x_bf16 = a.x_bf16 ? 1 : 0;
-    p.mode = a.mode;
-    p.norm_weight = a.norm_weight;
-    p.eps = a.eps;
-    p.k = a.k;
-    p.nsb = a.k / kSuperBlock;
-    p.members = a.members;
+    const ImmaParams p = params_of(a);
     return launch_kernel(gemv_imma_image_kernel, dim3((p.nsb + 7) / 8, a.members), dim3(256), 0, a.stream, p, static_cast<uint8_t*>(image));
 }
 
 cudaError_t launch_gemv_imma(const MmaGemvArgs& a) {
+    const Fetch fetch = fetch_of(a.value_type, a.k);
     switch (a.value_type) {
-        case kQ4_K: return launch_format<kQ4_K>(a);
-        case kQ5_K: return launch_format<kQ5_K>(a);
-        case kQ6_K: return launch_format<kQ6_K>(a);
+        case kQ4_K: return launch_format<kQ4_K, kBoxes>(a);
+        case kQ5_K: return launch_format<kQ5_K, kBoxes>(a);
+        case kQ6_K:
+            return fetch == kBoxes      ? launch_format<kQ6_K, kBoxes>(a)
+                   : fetch == kRowsEven ? launch_format<kQ6_K, kRowsEven>(a)
+                                        : launch_format<kQ6_K, kRowsOdd>(a);
+        case kQ8_0: return fetch == kBoxes ? launch_format<kQ8_0, kBoxes>(a) : launch_format<kQ8_0, kRowsOdd>(a);
         default: return cudaErrorInvalidValue;
     }
 }

@@ -78,6 +78,32 @@ __device__ __forceinline__ bool mbar_wait_bounded_hint(uint64_t* bar, uint32_t p
     return false;
 }
 
+// Bounded wait that polls without suspending: a thread that mbarrier.try_wait suspends is late by some hundred clocks, which the
+// hand-overs of a K step cannot afford.  `polls`: how often at most, kPolls (about a second) or nothing once a wait has run out.
+constexpr uint32_t kPolls = 1u << 26;
+__device__ __forceinline__ bool mbar_spin(uint32_t bar, uint32_t parity, uint32_t polls) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, q;\n\t"
+        ".reg .u32 left;\n\t"
+        "mov.u32 left, %3;\n\t"
+        "POLL:\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "@p bra DONE;\n\t"
+        "sub.u32 left, left, 1;\n\t"
+        "setp.gt.s32 q, left, 0;\n\t"
+        "@q bra POLL;\n\t"
+        "DONE:\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t"
+        "}"
+        : "=r"(done)
+        : "r"(bar), "r"(parity), "r"(polls)
+        : "memory");
+    return done != 0;
+}
+__device__ __forceinline__ bool mbar_spin(uint64_t* bar, uint32_t parity) { return mbar_spin(smem_addr(bar), parity, kPolls); }
+
 // Untiled bulk copy global -> shared of `bytes` (a multiple of 16; both
 // addresses 16-byte aligned), completion counted on `bar` in bytes.
 __device__ __forceinline__ void bulk_copy_g2s(void* dst_smem, const void* src_global, uint32_t bytes, uint64_t* bar) {

@@ -168,32 +168,6 @@ __device__ __forceinline__ uint32_t acc_column(int nt, int buffer, int sum) {
 }
 constexpr uint32_t kARing = kMaxTokens;   // first TMEM column of the A ring
 
-// Bounded wait that polls without suspending: a thread that mbarrier.try_wait suspends is late by some hundred clocks, which the
-// hand-overs of a K step cannot afford.  `polls`: how often at most, kPolls (about a second) or nothing once a wait has run out.
-constexpr uint32_t kPolls = 1u << 26;
-__device__ __forceinline__ bool mbar_spin(uint32_t bar, uint32_t parity, uint32_t polls) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p, q;\n\t"
-        ".reg .u32 left;\n\t"
-        "mov.u32 left, %3;\n\t"
-        "POLL:\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "@p bra DONE;\n\t"
-        "sub.u32 left, left, 1;\n\t"
-        "setp.gt.s32 q, left, 0;\n\t"
-        "@q bra POLL;\n\t"
-        "DONE:\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t"
-        "}"
-        : "=r"(done)
-        : "r"(bar), "r"(parity), "r"(polls)
-        : "memory");
-    return done != 0;
-}
-__device__ __forceinline__ bool mbar_spin(uint64_t* bar, uint32_t parity) { return mbar_spin(smem_addr(bar), parity, kPolls); }
-
 // ---------------------------------------------------------------- pair primitives
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");

@@ -472,3 +472,24 @@ def test_non_finite_activations_reach_the_output(ctx):
     engine_b200.CudaQ4KGemv.from_context(ctx).execute_warp(weight, xd.reshape(-1), yd)
     ctx.synchronize()
     assert not torch.isfinite(yd).any()
+
+
+# the edges of the narrow kernel's work split: fewer rows than a tile per SM, one tile and two tiles per CTA with a ragged end, many
+# one-chunk tiles (every sum slot in turn), one and two row-wise fetches per stage, Q8_0 rows that end inside a group of eight blocks
+@pytest.mark.parametrize("vt,n,k", [(8, 16, 32), (8, 257, 2048), (8, 5003, 1056), (8, 4800, 8192 + 96), (12, 17, 256), (12, 30011, 256),
+                                    (13, 2400, 2560), (14, 129, 256 * 21), (14, 5009, 256 * 10), (14, 20011, 256), (14, 4736, 2048)])
+@pytest.mark.parametrize("members", [1, 3, 8])
+def test_narrow_kernel_edges(ctx, gemv_path, vt, n, k, members):
+    if gemv_path != 0:
+        pytest.skip("the default path")
+    weight = upload(ctx, vt, synth.random_weight(vt, k, n, seed=n + k), k, n)
+    x = np.random.default_rng(members).standard_normal((members, k)).astype(np.float32)
+    y, x_seen = run_gemv(ctx, vt, weight, x, n)
+    exact = torch.empty(n, k, device=ctx.device)
+    engine_b200.dequantize(ctx, weight, exact)
+    ctx.synchronize()
+    seen = torch.from_numpy(x_seen).to(ctx.device).double()
+    expected = (seen @ exact.double().T).cpu().numpy()
+    scale = torch.sqrt(seen.square() @ exact.double().square().T).cpu().numpy()
+    # exact weights and 22-bit activations (15-bit ones where eight long rows do not fit the kernel): far inside the bound of the path
+    assert np.all(np.abs(y - expected) <= (1e-5 if members * k <= 65536 else 1e-3) * np.maximum(np.abs(expected), scale))
