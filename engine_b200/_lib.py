@@ -194,3 +194,15 @@ def load() -> ctypes.CDLL:
         fn.argtypes = argtypes
     _lib = lib
     return lib
+
+
+def load_call():
+    """The extension module _call (csrc/call.c), the short way into ribn_gemv."""
+    import torch
+
+    try:
+        from . import _call
+    except ImportError as exc:
+        raise ImportError("engine_b200._call is missing. Build it with `python -m engine_b200.build`") from exc
+    _call.set_dtypes(torch.float32, torch.bfloat16)
+    return _call

@@ -1,7 +1,8 @@
 """Ahead-of-time build of libribn_b200.so for sm_100a with nvcc (no JIT, no run-time compile).
 
 `python -m engine_b200.build` compiles every .cu under csrc/ and links the shared library
-in-tree, next to this file, where the ctypes loader looks for it.
+in-tree, next to this file, where the ctypes loader looks for it, and csrc/call.c as the
+extension module _call, the short way into ribn_gemv.
 """
 from __future__ import annotations
 
@@ -10,11 +11,13 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libribn_b200.so")
+CALL = os.path.join(HERE, "_call" + sysconfig.get_config_var("EXT_SUFFIX"))
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 # No --use_fast_math: flush-to-zero or approximate division would break bit-exact dequantisation.
@@ -41,7 +44,7 @@ def _newest_input() -> float:
 
 
 def build(force: bool = False, verbose: bool = False, extra: list[str] | None = None) -> str:
-    if not force and os.path.exists(LIB) and os.path.getmtime(LIB) >= _newest_input():
+    if not force and all(os.path.exists(p) and os.path.getmtime(p) >= _newest_input() for p in (LIB, CALL)):
         return LIB
     os.makedirs(OBJ, exist_ok=True)
     compiler = nvcc()
@@ -62,6 +65,8 @@ def build(force: bool = False, verbose: bool = False, extra: list[str] | None = 
     link = [compiler, *ARCH, "-shared", "-cudart", "shared", "-o", LIB, *objects,
             "-Xlinker", "-rpath,/usr/local/cuda/lib64"]
     subprocess.run(link, check=True)
+    subprocess.run([os.environ.get("CC", "gcc"), "-O2", "-shared", "-fPIC", "-Wall", "-I", sysconfig.get_paths()["include"],
+                    os.path.join(CSRC, "call.c"), "-o", CALL], check=True)
     return LIB
 
 

@@ -76,11 +76,15 @@ class RibnContext:
         if status != _lib.RIBN_OK:
             raise CudaQuantizedKernelError(status, "ribn_create failed (an sm_100 GPU is required)")
         self.handle = handle
+        self._address = handle.value   # for the calls that do not go through ctypes; 0 once closed
+        self._gemv_address = ctypes.cast(self._lib.ribn_gemv, ctypes.c_void_p).value
+        self._call_gemv = _lib.load_call().gemv
 
     def close(self) -> None:
         if getattr(self, "handle", None):
             self._lib.ribn_destroy(self.handle)
             self.handle = None
+            self._address = 0
 
     def __del__(self):
         try:
@@ -132,6 +136,7 @@ class CudaQuantizedWeight:
         self._value_type = int(value_type)
         self._encoded = encoded
         self._descriptor = None
+        self._descriptor_address = 0
 
     def spec(self) -> WeightTensorSpec:
         return self._spec
@@ -150,6 +155,7 @@ class CudaQuantizedWeight:
             dims = (ctypes.c_uint64 * 4)(*(list(self._spec.dimensions)[:4] + [0] * (4 - min(4, len(self._spec.dimensions)))))
             self._descriptor = QWeight(self._encoded.data_ptr(), self._encoded.numel(), self._value_type,
                                        len(self._spec.dimensions), dims)
+            self._descriptor_address = ctypes.addressof(self._descriptor)
         return self._descriptor
 
 
@@ -204,9 +210,10 @@ class _CudaQuantizedGemv:
 
     def _run(self, weight: CudaQuantizedWeight, x: torch.Tensor, y: torch.Tensor, members: int) -> None:
         ctx = self.context
-        descriptor = weight.descriptor()
-        ctx.check(ctx._lib.ribn_gemv(ctx.handle, self.VALUE_TYPE, ctypes.byref(descriptor), x.data_ptr(), _dtype_code(x),
-                                     x.numel(), y.data_ptr(), _dtype_code(y), y.numel(), members))
+        descriptor = weight._descriptor_address or ctypes.addressof(weight.descriptor())
+        status = ctx._call_gemv(ctx._gemv_address, ctx._address, self.VALUE_TYPE, descriptor, x, y, members)
+        if status:
+            ctx.check(status)
 
     def execute(self, weight: CudaQuantizedWeight, input: torch.Tensor, output: torch.Tensor) -> None:
         """quantized.rs:1612: one matrix-vector product; asynchronous on the context's stream."""
