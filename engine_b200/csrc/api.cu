@@ -414,8 +414,12 @@ int enqueue_mma(ribn_ctx* ctx, const ribn_qweight* w, uint64_t k, uint64_t n, co
             a.device_status = ctx->device_status;
             a.sm_count = ctx->sm_count;
             a.stream = ctx->stream;
-            const bool wide = a.members >= ctx->mma_image_members || (a.members <= 2 && ctx->mma_image_members <= 3 && a.k / 256 > 24) ||
-                              (shared_image && a.members >= 2 && ctx->mma_image_members <= 8) || (mode == 2 && ctx->mma_image_members <= 8);
+            // Every CTA converts the activations itself while that is at most about two slices per warp (measured, 3 x 2048: 7.5 -> 5.0
+            // us without the pre-pass, 3 x 4096 and 2 x 8192 slower); several projections of one normalised or gated input of two rows or
+            // more share the image, and silu(gate) * up is worth making once.
+            const bool by_size = static_cast<uint64_t>(a.members) * ((a.k + 255) / 256) > 40;
+            const bool wide = ctx->mma_image_members > 8 ? false
+                              : (ctx->mma_image_members == 3 ? by_size : a.members >= ctx->mma_image_members) || (shared_image && a.members >= 2) || mode == 2;
             const uint64_t image_bytes = ribn::gemv_imma_image_bytes(a.members, a.k);
             if (wide && offset + image_bytes <= ctx->workspace_bytes) {
                 void* image = static_cast<uint8_t*>(ctx->workspace) + offset;

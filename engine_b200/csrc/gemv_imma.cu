@@ -34,6 +34,8 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <algorithm>
+
 #include "formats.cuh"
 #include "internal.h"
 #include "pack_activations.cuh"
@@ -51,7 +53,7 @@ constexpr int kConsumerWarps = kGroups * kGroupWarps;
 constexpr int kConsumers = kConsumerWarps * 32;
 constexpr int kThreads = kConsumers + 32;      // + the producer warp
 constexpr int kTileRows = 16;                  // weight rows per tile (the M of m16n8k32)
-constexpr int kMaxStages = 8;
+constexpr int kMaxStages = 8;                // of a CTA: one ring when it has one tile, else two (one per group) of half as many
 constexpr int kMaxSlots = 5;                   // tiles of a group whose partial sums may be waiting for their finisher
 constexpr int kMaxMembers = 8;                 // four column groups of two members
 constexpr int kSliceBytes = 768;               // image bytes per (member, super-block): 8 sub-blocks x 3 planes x 32
@@ -97,7 +99,8 @@ struct ImmaParams {
     void* y;
     int y_bf16;
     int accumulate;
-    int k, n, nsb, members, stages;
+    int k, n, nsb, members;
+    int stages, rings;          // stages per ring, and rings (1 when no CTA has a second tile)
     int slots;                  // partial-sum slots per consumer group
     int tile_quotient, tile_remainder;   // tiles per CTA, and how many CTAs have one more
     int* status;
@@ -548,13 +551,14 @@ __host__ __device__ inline size_t imma_fixed_bytes(int members, int nsb, int slo
 }
 
 // Where a CTA's stream of stages goes: chunk c (eight super-blocks) of its tiles, pairs of tiles interleaved chunk by chunk,
-// group g taking tile 2 i + g; an odd last tile is group 0's alone.
+// group g taking tile 2 i + g; an odd last tile is group 0's alone.  Each group has a ring of its own: a wait on one parity bit
+// is only safe for a warp that sees every phase of the barrier.
 struct Walk {
-    int stage, phase;
-    __device__ __forceinline__ void step(int items, int stages) {
-        stage += items;
-        if (stage >= stages) {
-            stage -= stages;
+    int first, stage, phase;
+    __device__ __forceinline__ int slot() const { return first + stage; }
+    __device__ __forceinline__ void step(int stages) {
+        if (++stage == stages) {
+            stage = 0;
             phase ^= 1;
         }
     }
@@ -567,7 +571,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_imma_kernel(const __grid_con
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((128u - (smem_addr(smem_raw) & 127u)) & 127u);
     uint8_t* ring = smem;
-    uint8_t* zeros = ring + static_cast<size_t>(p.stages) * P::kStageBytes;
+    uint8_t* zeros = ring + static_cast<size_t>(p.stages * p.rings) * P::kStageBytes;
     uint8_t* image = zeros + kZeroBytes;
     uint8_t* planes = image;
     __half* sums = reinterpret_cast<__half*>(planes + image_plane_bytes(p.members, p.nsb));
@@ -604,16 +608,17 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_imma_kernel(const __grid_con
 
     if (warp == kConsumerWarps) {
         // ---------------- producer warp: the weight stream does not depend on the activations ----------------
-        Walk walk{0, 1};   // the first round of every stage waits for nothing: parity 1 of a fresh barrier has passed
+        // the first round of every stage waits for nothing: parity 1 of a fresh barrier has passed
+        Walk walk{0, 0, 1}, other{stages, 0, 1};
         auto request = [&](int tile, int chunk) {
-            if (lane == 0 || FETCH != kBoxes) ok = ok && mbar_spin(&empty[walk.stage], walk.phase);
+            if (lane == 0 || FETCH != kBoxes) ok = ok && mbar_spin(&empty[walk.slot()], walk.phase);
             if (FETCH != kBoxes) ok = __all_sync(0xffffffffu, ok);
             if (ok) {
                 const int row0 = (tile_begin + tile) * kTileRows;
                 const int sbs = min(kGroupWarps, p.nsb - chunk * kGroupWarps);
                 const int boxes = (sbs + P::kBoxSb - 1) / P::kBoxSb;
-                uint8_t* stage = ring + static_cast<size_t>(walk.stage) * P::kStageBytes;
-                uint64_t* bar = &full[walk.stage];
+                uint8_t* stage = ring + static_cast<size_t>(walk.slot()) * P::kStageBytes;
+                uint64_t* bar = &full[walk.slot()];
                 if constexpr (FETCH == kBoxes) {
                     if (lane == 0) {
                         mbar_arrive_expect_tx(bar, static_cast<uint32_t>(boxes * P::kBoxBytes));
@@ -636,15 +641,21 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_imma_kernel(const __grid_con
                     if (mine) bulk_copy_g2s(stage + b * P::kBoxBytes + row * P::kRowPitch, p.weights + first, bytes, bar);
                 }
             }
-            walk.step(1, stages);
+            walk.step(stages);
         };
 #pragma unroll 1
         for (int tile = 0; tile < tiles; tile += 2) {
             const int both = tile + 1 < tiles ? 2 : 1;
 #pragma unroll 1
-            for (int chunk = 0; chunk < chunks; ++chunk) {
-                request(tile, chunk);
-                if (both == 2) request(tile + 1, chunk);
+            for (int step = 0; step < both * chunks; ++step) {
+                if (both == 1) {
+                    request(tile, step);
+                } else {
+                    request(tile + (step & 1), step >> 1);
+                    const Walk next = other;
+                    other = walk;
+                    walk = next;
+                }
             }
         }
         ok = __all_sync(0xffffffffu, ok);
@@ -729,8 +740,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_imma_kernel(const __grid_con
         // This warp's super-block inside a stage: box w8 / kBoxSb, position w8 % kBoxSb, rows g and g + 8.
         const uint32_t ring_addr = smem_addr(ring) + static_cast<uint32_t>((w8 / P::kBoxSb) * P::kBoxBytes + (w8 % P::kBoxSb) * P::kSbBytes + g * P::kRowPitch);
         lx.advance(w8);   // the warp's super-block of the first chunk
-        Walk walk{0, 0};
-        walk.step(tiles > 1 ? group : 0, stages);
+        Walk walk{group * stages, 0, 0};
         int slot = 0, slot_phase = 0, turn = 0;   // of the group's next tile: where its sums meet, and which warp finishes it
 
 #pragma unroll 1
@@ -739,7 +749,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_imma_kernel(const __grid_con
             float acc[GROUPS][2], mins[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
             for (int q = 0; q < GROUPS; ++q) acc[q][0] = acc[q][1] = 0.0f;
-            const int items = (tile | 1) < tiles ? kGroups : 1;   // stages from one chunk of this tile to its next
             uint32_t delta0 = 0u, delta1 = 0u;   // how far behind the copied boundary the rows start
             if (FETCH != kBoxes) {
                 delta0 = static_cast<uint32_t>(static_cast<unsigned long long>(row0 + g) * p.row_bytes) & 15u;
@@ -747,10 +756,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_imma_kernel(const __grid_con
             }
 #pragma unroll 1
             for (int chunk = 0; chunk < chunks; ++chunk) {
-                ok = ok && mbar_spin(&full[walk.stage], walk.phase);
+                ok = ok && mbar_spin(&full[walk.slot()], walk.phase);
                 const int sb = chunk * kGroupWarps + w8;
                 if (sb < p.nsb) {
-                    const uint32_t base = ring_addr + static_cast<uint32_t>(walk.stage) * P::kStageBytes;
+                    const uint32_t base = ring_addr + static_cast<uint32_t>(walk.slot()) * P::kStageBytes;
                     const uint32_t p0 = base + delta0, p1 = base + 8 * P::kRowPitch + delta1;
                     if constexpr (FMT == kQ6_K) {
                         // 210-byte super-blocks: in rows that start on a word the warp's one does when its position in the box is even
@@ -765,9 +774,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_imma_kernel(const __grid_con
                 }
                 lx.advance(kGroupWarps);
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&empty[walk.stage]);
-                // behind the tile's last chunk: the first of the group's next tile is one full pair's stride on
-                walk.step(items, stages);
+                if (lane == 0) mbar_arrive(&empty[walk.slot()]);
+                walk.step(stages);
             }
             lx.advance(-chunks * kGroupWarps);
             // Tile end: a member's two plane shares sit in neighbouring lanes and its minima in lane q of the four; the eight warps'
@@ -880,21 +888,22 @@ Fetch fetch_of(uint32_t value_type, int k) {
     return row % 4 == 0 && value_type == kQ6_K ? kRowsEven : kRowsOdd;
 }
 
-// Stages and slots of a launch; stages = 0 when fewer than two fit.
+// Rings, stages per ring and slots of a launch; stages = 0 when two stages do not fit.
 struct Ring {
-    int stages, slots;
+    int rings, stages, slots;
 };
-Ring ring_of(size_t stage_bytes, int members, int nsb, int items, int wanted) {
+Ring ring_of(size_t stage_bytes, int members, int nsb, int tiles_per_cta, int wanted) {
     const int chunks = (nsb + kGroupWarps - 1) / kGroupWarps;
-    for (int stages = kMaxStages; stages >= 2; --stages) {
-        if (wanted > 0 && stages > wanted && stages > 2) continue;
-        if (stages > 2 && stages > items) continue;   // no more than the CTA has use for
-        // A warp that writes the slot of the group's tile T + slots has seen its last stage, and every warp of the group has given
-        // back all stages of the ring's length earlier; the first stage of tile T + 1 must be among them.
-        const int slots = 1 + (stages + 1 > chunks ? (stages + 1 - chunks + 2 * chunks - 1) / (2 * chunks) : 0);
-        if (imma_fixed_bytes(members, nsb, slots) + stages * stage_bytes <= kSmemLimit) return Ring{stages, slots};
+    const int rings = tiles_per_cta > 1 ? 2 : 1, least = 2 / rings;
+    const int most = std::min(kMaxStages / rings, std::max(least, chunks * ((tiles_per_cta + 1) / 2)));   // no more than the CTA has use for
+    for (int stages = most; stages >= least; --stages) {
+        if (wanted > 0 && stages * rings > wanted && stages > least) continue;
+        // A warp that writes the slot of its group's tile T + slots has seen that tile's last stage, for which every warp of the group
+        // gave the stage's last use back; that use is of tile T + 1 or later, begun when the sums of tile T were complete.
+        const int slots = (stages + chunks) / chunks;
+        if (imma_fixed_bytes(members, nsb, slots) + static_cast<size_t>(stages * rings) * stage_bytes <= kSmemLimit) return Ring{rings, stages, slots};
     }
-    return Ring{0, 0};
+    return Ring{0, 0, 0};
 }
 size_t stage_bytes_of(uint32_t value_type, Fetch fetch) {
     switch (value_type) {
@@ -926,16 +935,16 @@ cudaError_t launch_groups(const MmaGemvArgs& a) {
     ImmaParams p = params_of(a);
     // One CTA per SM: its sixteen consumer warps share one image of the activations, and whole SMs divide the tiles more
     // evenly than halves do.
-    const int tiles = (a.n + kTileRows - 1) / kTileRows, chunks = (p.nsb + kGroupWarps - 1) / kGroupWarps;
+    const int tiles = (a.n + kTileRows - 1) / kTileRows;
     const int grid = tiles < a.sm_count ? tiles : a.sm_count;
     p.tile_quotient = tiles / grid;
     p.tile_remainder = tiles % grid;
-    const int items = (p.tile_quotient + (p.tile_remainder > 0 ? 1 : 0)) * chunks;
-    const Ring ring = ring_of(P::kStageBytes, a.members, p.nsb, items, a.stages);
+    const Ring ring = ring_of(P::kStageBytes, a.members, p.nsb, p.tile_quotient + (p.tile_remainder > 0 ? 1 : 0), a.stages);
     if (ring.stages == 0) return cudaErrorInvalidConfiguration;
     p.stages = ring.stages;
+    p.rings = ring.rings;
     p.slots = ring.slots;
-    const size_t smem = imma_fixed_bytes(a.members, p.nsb, p.slots) + static_cast<size_t>(p.stages) * P::kStageBytes;
+    const size_t smem = imma_fixed_bytes(a.members, p.nsb, p.slots) + static_cast<size_t>(p.stages * p.rings) * P::kStageBytes;
     static int configured_device = -1;
     int device = 0;
     cudaGetDevice(&device);
