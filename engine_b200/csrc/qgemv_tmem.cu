@@ -60,10 +60,6 @@
 namespace ribn {
 namespace {
 
-// Upper bound of one suspended poll of an mbarrier wait: a waiting thread wakes when the phase completes, and until then
-// takes no issue slots from the threads that unpack.
-constexpr uint32_t kWaitHintNs = 1000u;
-
 constexpr int kRows = 128;                 // weight rows per CTA = UMMA M = TMEM lanes
 constexpr int kWorkerWarps = 8;
 constexpr int kWorkers = kWorkerWarps * 32;
@@ -81,6 +77,15 @@ struct Roles {
 constexpr int kPairs = 4;                  // 64-weight pairs of sub-blocks per super-block = A slots in TMEM
 constexpr int kPairColumns = 32;           // TMEM columns of one pair: 64 halves per row
 constexpr int kMaxStages = 4;
+
+// The hand-overs between workers and issuers poll: a suspended thread wakes some hundred clocks late.  So do waits for memory, except
+// where sixteen worker warps share the SM: there a suspended thread leaves its issue slots to those that unpack.  (A decode
+// step of 32 rows, eight layers: 1474 us with suspended waits, 1404 with polls.)
+constexpr uint32_t kWaitHintNs = 1000u;
+template <int NT>
+__device__ __forceinline__ bool memory_wait(uint64_t* bar, uint32_t parity) {
+    return NT >= 64 ? mbar_wait_bounded_hint(bar, parity, kWaitHintNs) : mbar_spin(bar, parity);
+}
 
 // Tiled TMA wants a 16-byte aligned base and row pitch.  A Q6_K matrix whose rows are 210 * nsb bytes with nsb not a
 // multiple of eight has neither for most rows, but rows n, n + P, n + 2 P, ... (P = 16 / gcd(row bytes, 16)) are P * row
@@ -587,7 +592,7 @@ __global__ void __launch_bounds__(Roles<NT>::kThreads, NT >= 64 ? 1 : 2) qgemv_t
         bool ok = true;
         for (int i = 0; i < local_sb && ok; ++i) {
             const int bs = i % p.b_stages;
-            ok = __all_sync(0xffffffffu, mbar_wait_bounded_hint(&b_full[bs], (i / p.b_stages) & 1, kWaitHintNs));
+            ok = __all_sync(0xffffffffu, memory_wait<NT>(&b_full[bs], (i / p.b_stages) & 1));
             if (!ok) break;
             if (i < 4 && which == 0) stamp(p, 1, i * 4);
             const uint64_t desc_b0 = umma_smem_desc_sw128(smem_addr(b_ring + static_cast<size_t>(bs) * I::kStageBytes));
@@ -595,7 +600,7 @@ __global__ void __launch_bounds__(Roles<NT>::kThreads, NT >= 64 ? 1 : 2) qgemv_t
 #pragma unroll
             for (int jj = 0; jj < 2; ++jj) {
                 const int j = which * 2 + jj;
-                ok = ok && __all_sync(0xffffffffu, mbar_wait_bounded_hint(&a_full[abuf * kPairs + j], (i / AB) & 1, kWaitHintNs));
+                ok = ok && __all_sync(0xffffffffu, mbar_spin(&a_full[abuf * kPairs + j], (i / AB) & 1));
                 if (!ok) break;
                 if (i < 4 && which == 0) stamp(p, 1, i * 4 + 1 + jj);
                 tcgen05_fence_after_sync();
@@ -607,7 +612,7 @@ __global__ void __launch_bounds__(Roles<NT>::kThreads, NT >= 64 ? 1 : 2) qgemv_t
             if (!ok) break;
             if (FMT != kQ6_K && which == 0) {
                 // minimum term: A = -dmin * m[g] twice (K slots 0..7 meet the block sums' hi parts, 8..15 their lo parts)
-                ok = __all_sync(0xffffffffu, mbar_wait_bounded_hint(&min_full[i & 1], (i >> 1) & 1, kWaitHintNs));
+                ok = __all_sync(0xffffffffu, mbar_spin(&min_full[i & 1], (i >> 1) & 1));
                 if (!ok) break;
                 tcgen05_fence_after_sync();
                 umma_f16_tmem_a_elected(d_tmem, tmem_base + P::kColAMin + (i & 1) * 8, desc_b0 + static_cast<uint64_t>(4 * (I::kTileBytes >> 4)), idesc, 1u);
@@ -633,7 +638,7 @@ __global__ void __launch_bounds__(Roles<NT>::kThreads, NT >= 64 ? 1 : 2) qgemv_t
 #pragma unroll 1
         for (int i = set; i < local_sb; i += kSets) {
             const int s = i % p.raw_stages;
-            if (ok && !mbar_wait_bounded_hint(&raw_full[s], (i / p.raw_stages) & 1, kWaitHintNs)) {
+            if (ok && !memory_wait<NT>(&raw_full[s], (i / p.raw_stages) & 1)) {
                 atomicExch(p.status, kDeviceWaitTimeout);
                 ok = false;
             }
@@ -668,7 +673,7 @@ __global__ void __launch_bounds__(Roles<NT>::kThreads, NT >= 64 ? 1 : 2) qgemv_t
                             out_hi[r] = hmul2(out_hi[r], d2);
                         }
                     }
-                    if (i >= AB && ok && !mbar_wait_bounded_hint(&a_empty[slot], ((i / AB) - 1) & 1, kWaitHintNs)) {
+                    if (i >= AB && ok && !mbar_spin(&a_empty[slot], ((i / AB) - 1) & 1)) {
                         atomicExch(p.status, kDeviceWaitTimeout);
                         ok = false;
                     }
@@ -700,7 +705,7 @@ __global__ void __launch_bounds__(Roles<NT>::kThreads, NT >= 64 ? 1 : 2) qgemv_t
                 mins[2] = half2_bits(nd * byte_of(m_hi, 0), nd * byte_of(m_hi, 1));
                 mins[3] = half2_bits(nd * byte_of(m_hi, 2), nd * byte_of(m_hi, 3));
                 mins[4] = mins[0]; mins[5] = mins[1]; mins[6] = mins[2]; mins[7] = mins[3];
-                if (i >= 2 && ok && !mbar_wait_bounded_hint(&min_empty[i & 1], ((i >> 1) - 1) & 1, kWaitHintNs)) {
+                if (i >= 2 && ok && !mbar_spin(&min_empty[i & 1], ((i >> 1) - 1) & 1)) {
                     atomicExch(p.status, kDeviceWaitTimeout);
                     ok = false;
                 }
@@ -726,7 +731,7 @@ __global__ void __launch_bounds__(Roles<NT>::kThreads, NT >= 64 ? 1 : 2) qgemv_t
                         out_hi[r] = hmul2(out_hi[r], d2);
                     }
                 }
-                if (i >= AB && ok && !mbar_wait_bounded_hint(&a_empty[slot], ((i / AB) - 1) & 1, kWaitHintNs)) {
+                if (i >= AB && ok && !mbar_spin(&a_empty[slot], ((i / AB) - 1) & 1)) {
                     atomicExch(p.status, kDeviceWaitTimeout);
                     ok = false;
                 }
@@ -749,7 +754,7 @@ __global__ void __launch_bounds__(Roles<NT>::kThreads, NT >= 64 ? 1 : 2) qgemv_t
         if (set == 0) {
         pdl_wait_prior();   // the scale factors (and y, when it is accumulated into) come from earlier kernels
         if (threadIdx.x < NT) up[threadIdx.x] = reinterpret_cast<const float*>(p.image + I::scales_offset(p.nsb))[threadIdx.x];
-        if (ok && !mbar_wait_bounded_hint(d_full, 0, kWaitHintNs)) {
+        if (ok && !mbar_spin(d_full, 0)) {
             atomicExch(p.status, kDeviceWaitTimeout);
             ok = false;
         }
@@ -839,6 +844,10 @@ __global__ void __launch_bounds__(Roles<NT>::kThreads, NT >= 64 ? 1 : 2) qgemv_t
                 first_item = static_cast<int>(static_cast<long long>(items) * blockIdx.y / p.ksplit);
                 last_item = static_cast<int>(static_cast<long long>(items) * (blockIdx.y + 1) / p.ksplit);
             }
+            // Every CTA that has seen all partial tiles departs; the last one resets both counters.  Counted here, so that the
+            // answer is back by the time the sum is done.
+            unsigned int departure = 0;
+            if (p.cooperative && threadIdx.x == 0) departure = atomicAdd(departed, 1u);
             if (*last_flag != 0) {
                 __threadfence();
                 const size_t plane = static_cast<size_t>(p.members) * p.n;
@@ -884,13 +893,9 @@ __global__ void __launch_bounds__(Roles<NT>::kThreads, NT >= 64 ? 1 : 2) qgemv_t
                     }
                 }
             }
-            if (p.cooperative) {
-                // the last CTA to leave resets both counters: by then every CTA of the row tile has passed its wait
-                named_barrier_sync(1, kWorkers);
-                if (threadIdx.x == 0 && atomicAdd(departed, 1u) == static_cast<unsigned int>(p.ksplit - 1)) {
-                    *departed = 0;
-                    *ticket = 0;
-                }
+            if (p.cooperative && threadIdx.x == 0 && departure == static_cast<unsigned int>(p.ksplit - 1)) {
+                *departed = 0;
+                *ticket = 0;
             }
         }
         }   // first worker set
