@@ -759,7 +759,7 @@ def main() -> None:
     step_bytes = sum(case_bytes(*c) for c in cases)
     # Launches per call: one for up to two member rows over at most 24 super-blocks (the kernel converts its activations
     # itself), otherwise an activation pre-pass and the GEMV kernel.
-    launches_per_step = sum(1 if (m <= 2 and k // 256 <= 24) else 2 for _, _, k, m in cases)
+    launches_per_step = sum(1 if m * (k // 256) <= 40 else 2 for _, _, k, m in cases)
 
     def launch(vt, n, k, m):
         ring = rings[(vt, n, k)]

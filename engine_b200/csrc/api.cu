@@ -377,60 +377,73 @@ bool mma_serves(const ribn_ctx* ctx, const ribn_qweight* w, uint64_t k, uint64_t
     return ribn::gemv_mma_supports(w->value_type, static_cast<int>(k), static_cast<int>(n), per_launch, w->data);
 }
 
+// Arguments of the integer tensor-core kernel for rows m0 .. of a call.
+ribn::MmaGemvArgs imma_args(const ribn_ctx* ctx, const ribn_qweight* w, uint64_t k, uint64_t n, const void* x, int x_dtype, int mode,
+                            const float* norm_weight, float eps, void* y, int y_dtype, uint32_t members, bool accumulate, uint32_t m0) {
+    ribn::MmaGemvArgs a{};
+    a.weights = static_cast<const uint8_t*>(w->data);
+    a.value_type = w->value_type;
+    a.k = static_cast<int>(k);
+    a.n = static_cast<int>(n);
+    a.members = static_cast<int>(members - m0 < 8 ? members - m0 : 8);
+    a.x = static_cast<const uint8_t*>(x) + static_cast<uint64_t>(m0) * k * (mode == 2 ? 2 : 1) * dtype_bytes(x_dtype);
+    a.x_bf16 = x_dtype == RIBN_BF16;
+    a.mode = mode;
+    a.norm_weight = norm_weight;
+    a.eps = eps;
+    a.y = static_cast<uint8_t*>(y) + static_cast<uint64_t>(m0) * n * dtype_bytes(y_dtype);
+    a.y_bf16 = y_dtype == RIBN_BF16;
+    a.accumulate = accumulate;
+    a.stages = ctx->mma_stages;
+    a.device_status = ctx->device_status;
+    a.sm_count = ctx->sm_count;
+    a.stream = ctx->stream;
+    return a;
+}
+
+// Where the images of a call of that kernel start in the workspace: behind the ones the f16 kernel would keep for the same call.
+// Q8_0 rows may keep their images in an order of their own, behind the plain ones.
+uint64_t imma_image_offset(const ribn::MmaGemvArgs& a, uint32_t members) {
+    const uint64_t launches = (members + 7) / 8;
+    const int per_launch = members < 8 ? static_cast<int>(members) : 8;
+    uint64_t offset = launches * ribn::gemv_mma_image_bytes(per_launch, a.k, 2);
+    if (ribn::gemv_imma_rotates(a.value_type, a.k)) offset += launches * ribn::gemv_imma_image_bytes(per_launch, a.k);
+    return offset;
+}
+
+// Gives `a` its image when the call is to have one, made now unless `ready`.
+cudaError_t imma_image(const ribn_ctx* ctx, ribn::MmaGemvArgs& a, bool shared_image, bool ready, uint64_t& offset) {
+    // Every CTA converts the activations itself while that is at most about two slices per warp (measured, 3 x 2048: 7.5 -> 5.0
+    // us without the pre-pass, 3 x 4096 and 2 x 8192 slower); several projections of one normalised or gated input of two rows or
+    // more share the image, and silu(gate) * up is worth making once.
+    const bool by_size = static_cast<uint64_t>(a.members) * ((a.k + 255) / 256) > 40;
+    const bool wide = ctx->mma_image_members > 8 ? false
+                      : (ctx->mma_image_members == 3 ? by_size : a.members >= ctx->mma_image_members) || (shared_image && a.members >= 2) || a.mode == 2;
+    const uint64_t image_bytes = ribn::gemv_imma_image_bytes(a.members, a.k);
+    if (!wide || offset + image_bytes > ctx->workspace_bytes) return cudaSuccess;
+    void* image = static_cast<uint8_t*>(ctx->workspace) + offset;
+    offset += image_bytes;
+    a.image = image;
+    return ready ? cudaSuccess : ribn::launch_gemv_imma_image(a, image);
+}
+
 // `images_made` (fused calls: shared by the projections of one input): bit 0 = the f16 image of this x is in the
-// workspace, bit 1 = the int8 image is (the two narrow kernels keep different images, side by side).
+// workspace, bit 1 = the int8 image is (the two narrow kernels keep different images, side by side), bit 2 = the one of Q8_0.
 int enqueue_mma(ribn_ctx* ctx, const ribn_qweight* w, uint64_t k, uint64_t n, const void* x, int x_dtype, int mode, const float* norm_weight,
                 float eps, void* y, int y_dtype, uint32_t members, bool accumulate, unsigned* images_made, bool shared_image = false) {
     const bool x_bf16 = x_dtype == RIBN_BF16;
     const uint64_t x_row_bytes = k * (mode == 2 ? 2 : 1) * dtype_bytes(x_dtype);
     unsigned none_made = 0;
     if (images_made == nullptr) images_made = &none_made;
-    const uint32_t per_launch = members < 8 ? members : 8;
     if (imma_serves(ctx, w, k, n, members)) {
-        // its images follow the ones the f16 kernel would keep for the same call
-        uint64_t offset = static_cast<uint64_t>((members + 7) / 8) * ribn::gemv_mma_image_bytes(static_cast<int>(per_launch), static_cast<int>(k), 2);
-        // Q8_0 rows may keep their images in an order of their own, behind the plain ones
-        const bool rotated = ribn::gemv_imma_rotates(w->value_type, static_cast<int>(k));
-        const unsigned made = rotated ? 4u : 2u;
-        if (rotated) offset += static_cast<uint64_t>((members + 7) / 8) * ribn::gemv_imma_image_bytes(static_cast<int>(per_launch), static_cast<int>(k));
+        const unsigned made = ribn::gemv_imma_rotates(w->value_type, static_cast<int>(k)) ? 4u : 2u;
+        uint64_t offset = 0;
         for (uint32_t m0 = 0; m0 < members; m0 += 8) {
-            ribn::MmaGemvArgs a{};
-            a.weights = static_cast<const uint8_t*>(w->data);
-            a.value_type = w->value_type;
-            a.k = static_cast<int>(k);
-            a.n = static_cast<int>(n);
-            a.members = static_cast<int>(members - m0 < 8 ? members - m0 : 8);
-            a.x = static_cast<const uint8_t*>(x) + static_cast<uint64_t>(m0) * x_row_bytes;
-            a.x_bf16 = x_bf16;
-            a.mode = mode;
-            a.norm_weight = norm_weight;
-            a.eps = eps;
-            a.y = static_cast<uint8_t*>(y) + static_cast<uint64_t>(m0) * n * dtype_bytes(y_dtype);
-            a.y_bf16 = y_dtype == RIBN_BF16;
-            a.accumulate = accumulate;
-            a.stages = ctx->mma_stages;
-            a.resident = ctx->mma_resident;
-            a.grid_ctas = ctx->mma_ctas;
-            a.device_status = ctx->device_status;
-            a.sm_count = ctx->sm_count;
-            a.stream = ctx->stream;
-            // Every CTA converts the activations itself while that is at most about two slices per warp (measured, 3 x 2048: 7.5 -> 5.0
-            // us without the pre-pass, 3 x 4096 and 2 x 8192 slower); several projections of one normalised or gated input of two rows or
-            // more share the image, and silu(gate) * up is worth making once.
-            const bool by_size = static_cast<uint64_t>(a.members) * ((a.k + 255) / 256) > 40;
-            const bool wide = ctx->mma_image_members > 8 ? false
-                              : (ctx->mma_image_members == 3 ? by_size : a.members >= ctx->mma_image_members) || (shared_image && a.members >= 2) || mode == 2;
-            const uint64_t image_bytes = ribn::gemv_imma_image_bytes(a.members, a.k);
-            if (wide && offset + image_bytes <= ctx->workspace_bytes) {
-                void* image = static_cast<uint8_t*>(ctx->workspace) + offset;
-                offset += image_bytes;
-                if ((*images_made & made) == 0) {
-                    const cudaError_t e = ribn::launch_gemv_imma_image(a, image);
-                    if (e != cudaSuccess) return record_cuda(ctx, e, "activation image launch");
-                }
-                a.image = image;
-            }
-            const cudaError_t e = ribn::launch_gemv_imma(a);
+            ribn::MmaGemvArgs a = imma_args(ctx, w, k, n, x, x_dtype, mode, norm_weight, eps, y, y_dtype, members, accumulate, m0);
+            if (m0 == 0) offset = imma_image_offset(a, members);
+            cudaError_t e = imma_image(ctx, a, shared_image, (*images_made & made) != 0, offset);
+            if (e != cudaSuccess) return record_cuda(ctx, e, "activation image launch");
+            e = ribn::launch_gemv_imma(a);
             if (e != cudaSuccess) return record_cuda(ctx, e, "GEMV launch");
         }
         *images_made |= made;
@@ -661,9 +674,29 @@ int enqueue_fused(ribn_ctx* ctx, const ribn_gemv_job* jobs, uint32_t job_count, 
     if (all_mma) {
         const int mode = swiglu ? 2 : (norm_weight != nullptr ? 1 : 0);
         unsigned images_made = 0;
+        const bool shared_image = job_count > 1 && mode != 0;
         for (uint32_t j = 0; j < job_count; ++j) {
+            if (j + 1 < job_count && members <= 8 && imma_serves(ctx, jobs[j].weight, k, ns[j], members) &&
+                imma_serves(ctx, jobs[j + 1].weight, k, ns[j + 1], members)) {
+                // two projections whose formats have a kernel for both: one launch
+                ribn::MmaGemvArgs a = imma_args(ctx, jobs[j].weight, k, ns[j], x, x_dtype, mode, norm_weight, eps, jobs[j].y_device, jobs[j].y_dtype,
+                                                members, jobs[j].accumulate != 0, 0);
+                ribn::MmaGemvArgs b = imma_args(ctx, jobs[j + 1].weight, k, ns[j + 1], x, x_dtype, mode, norm_weight, eps, jobs[j + 1].y_device,
+                                                jobs[j + 1].y_dtype, members, jobs[j + 1].accumulate != 0, 0);
+                if (ribn::gemv_imma_pairs(a, b)) {
+                    uint64_t offset = imma_image_offset(a, members);
+                    cudaError_t e = imma_image(ctx, a, shared_image, (images_made & 2u) != 0, offset);
+                    if (e != cudaSuccess) return record_cuda(ctx, e, "activation image launch");
+                    b.image = a.image;
+                    images_made |= 2u;
+                    e = ribn::launch_gemv_imma_pair(a, b);
+                    if (e != cudaSuccess) return record_cuda(ctx, e, "GEMV launch");
+                    ++j;
+                    continue;
+                }
+            }
             const int rc = enqueue_mma(ctx, jobs[j].weight, k, ns[j], x, x_dtype, mode, norm_weight, eps, jobs[j].y_device, jobs[j].y_dtype, members,
-                                       jobs[j].accumulate != 0, &images_made, job_count > 1 && mode != 0);
+                                       jobs[j].accumulate != 0, &images_made, shared_image);
             if (rc != RIBN_OK) return rc;
         }
         return RIBN_OK;

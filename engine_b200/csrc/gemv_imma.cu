@@ -329,11 +329,15 @@ __device__ __forceinline__ void superblock(uint32_t p0, uint32_t p1, const LaneX
         f0 = lds64(p0 + 16 + 8 * t);
         f1 = lds64(p1 + 16 + 8 * t);
     }
-    int total[GROUPS][4];
+    // Q4_K, up to two column groups: the high nibbles go to the instruction where they stand, as sixteen times the quants, and their
+    // sums are kept apart (integers: 16 * low + high is sixteen times the sum, to the bit).  The logic pipe is what the loop is
+    // bound by, and the four shifts per pair were a sixth of its work.
+    constexpr bool kInPlace = FMT == kQ4_K && GROUPS <= 2;
+    int total[GROUPS][4], high[GROUPS][4];
 #pragma unroll
     for (int q = 0; q < GROUPS; ++q)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) total[q][i] = 0;
+        for (int i = 0; i < 4; ++i) total[q][i] = high[q][i] = 0;
 #define RIBN_IMMA_PAIR(G)                                                                                                      \
     {                                                                                                                          \
         const uint2 q0 = lds64(p0 + kQuantOffset + 32 * (G) + 8 * t), q1 = lds64(p1 + kQuantOffset + 32 * (G) + 8 * t);  \
@@ -345,27 +349,40 @@ __device__ __forceinline__ void superblock(uint32_t p0, uint32_t p1, const LaneX
             a3 = with_fifth<2 * (G)>(a3, f1.y);                                                                                \
         }                                                                                                                      \
         subblock<2 * (G), GROUPS>(a0, a1, a2, a3, lx, sc_lo0, sc_hi0, sc_lo1, sc_hi1, total);                                  \
-        a0 = (q0.x >> 4) & 0x0f0f0f0fu;                                                                                        \
-        a1 = (q1.x >> 4) & 0x0f0f0f0fu;                                                                                        \
-        a2 = (q0.y >> 4) & 0x0f0f0f0fu;                                                                                        \
-        a3 = (q1.y >> 4) & 0x0f0f0f0fu;                                                                                        \
+        if (kInPlace) {                                                                                                        \
+            a0 = q0.x & 0xf0f0f0f0u;                                                                                           \
+            a1 = q1.x & 0xf0f0f0f0u;                                                                                           \
+            a2 = q0.y & 0xf0f0f0f0u;                                                                                           \
+            a3 = q1.y & 0xf0f0f0f0u;                                                                                           \
+        } else {                                                                                                               \
+            a0 = (q0.x >> 4) & 0x0f0f0f0fu;                                                                                    \
+            a1 = (q1.x >> 4) & 0x0f0f0f0fu;                                                                                    \
+            a2 = (q0.y >> 4) & 0x0f0f0f0fu;                                                                                    \
+            a3 = (q1.y >> 4) & 0x0f0f0f0fu;                                                                                    \
+        }                                                                                                                      \
         if (FMT == kQ5_K) {                                                                                                    \
             a0 = with_fifth<2 * (G) + 1>(a0, f0.x);                                                                            \
             a1 = with_fifth<2 * (G) + 1>(a1, f1.x);                                                                            \
             a2 = with_fifth<2 * (G) + 1>(a2, f0.y);                                                                            \
             a3 = with_fifth<2 * (G) + 1>(a3, f1.y);                                                                            \
         }                                                                                                                      \
-        subblock<2 * (G) + 1, GROUPS>(a0, a1, a2, a3, lx, sc_lo0, sc_hi0, sc_lo1, sc_hi1, total);                              \
+        subblock<2 * (G) + 1, GROUPS>(a0, a1, a2, a3, lx, sc_lo0, sc_hi0, sc_lo1, sc_hi1, kInPlace ? high : total);                              \
     }
     RIBN_IMMA_PAIR(0)
     RIBN_IMMA_PAIR(1)
     RIBN_IMMA_PAIR(2)
     RIBN_IMMA_PAIR(3)
 #undef RIBN_IMMA_PAIR
+    if (kInPlace) {
+#pragma unroll
+        for (int q = 0; q < GROUPS; ++q)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) total[q][i] = 16 * total[q][i] + high[q][i];
+    }
     const float d0 = f16_bits_to_f32(h0.x & 0xffffu), dm0 = f16_bits_to_f32(h0.x >> 16);
     const float d1 = f16_bits_to_f32(h1.x & 0xffffu), dm1 = f16_bits_to_f32(h1.x >> 16);
     // Columns 2t, 2t+1 of a group: planes (p0, p1) of its first or second member for t = 0, 2; (p2, zeros) for t = 1, 3.
-    const float weight = (t & 1) ? 16384.0f : 1.0f;
+    const float weight = ((t & 1) ? 16384.0f : 1.0f) * (kInPlace ? 0.0625f : 1.0f);
 #pragma unroll
     for (int q = 0; q < GROUPS; ++q) {
         const float xs = __uint_as_float(lds32(lx.scale + 8 * q + 4 * (t >> 1))) * weight;
@@ -565,7 +582,7 @@ struct Walk {
 };
 
 template <uint32_t FMT, int FETCH, int GROUPS>
-__global__ void __launch_bounds__(kThreads, 1) gemv_imma_kernel(const __grid_constant__ CUtensorMap wmap, const ImmaParams p) {
+__device__ __forceinline__ void gemv_imma_body(const CUtensorMap& wmap, const ImmaParams& p, int cta) {
     using P = ImmaPlan<FMT, FETCH>;
     constexpr int kColumns = 2 * GROUPS;   // members of the column groups
     extern __shared__ uint8_t smem_raw[];
@@ -600,7 +617,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_imma_kernel(const __grid_con
         asm volatile("bar.arrive 2, %0;" ::"n"(kThreads) : "memory");
     }
 
-    const int cta = static_cast<int>(blockIdx.x);
     const int tile_begin = cta * p.tile_quotient + min(cta, p.tile_remainder);
     const int tiles = p.tile_quotient + (cta < p.tile_remainder ? 1 : 0);
     const int chunks = (p.nsb + kGroupWarps - 1) / kGroupWarps;
@@ -844,6 +860,23 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_imma_kernel(const __grid_con
     }
 }
 
+template <uint32_t FMT, int FETCH, int GROUPS>
+__global__ void __launch_bounds__(kThreads, 1) gemv_imma_kernel(const __grid_constant__ CUtensorMap wmap, const ImmaParams p) {
+    gemv_imma_body<FMT, FETCH, GROUPS>(wmap, p, static_cast<int>(blockIdx.x));
+}
+
+// Two projections of one input (a decode step's [q | k] and v) in one launch: the first `first_ctas` CTAs work on the first.
+// A small projection costs its start-up -- the end of the kernel before it, the conversion of the activations, the first
+// weights -- whatever its size: Q6_K 1024 x 4096 behind Q4_K 5120 x 4096 took 5.1 us, together they take no longer than
+// the first alone.
+template <uint32_t FMT1, uint32_t FMT2, int GROUPS>
+__global__ void __launch_bounds__(kThreads, 1) gemv_imma_pair_kernel(const __grid_constant__ CUtensorMap wmap1, const __grid_constant__ CUtensorMap wmap2,
+                                                                     const ImmaParams p1, const ImmaParams p2, int first_ctas) {
+    const int cta = static_cast<int>(blockIdx.x);
+    if (cta < first_ctas) gemv_imma_body<FMT1, kBoxes, GROUPS>(wmap1, p1, cta);
+    else gemv_imma_body<FMT2, kBoxes, GROUPS>(wmap2, p2, cta - first_ctas);
+}
+
 // ---------------------------------------------------------------- pre-pass: the activation image in global memory
 // grid (ceil(nsb / 8), members): warp w of CTA (c, m) converts super-block 8c + w of member row m.
 __global__ void __launch_bounds__(256) gemv_imma_image_kernel(const ImmaParams p, uint8_t* image) {
@@ -928,33 +961,21 @@ ImmaParams params_of(const MmaGemvArgs& a) {
     return p;
 }
 
-template <uint32_t FMT, int FETCH, int GROUPS>
-cudaError_t launch_groups(const MmaGemvArgs& a) {
+// Parameters, tensor map and shared memory of a call on `ctas` CTAs.
+template <uint32_t FMT, int FETCH>
+cudaError_t plan(const MmaGemvArgs& a, int ctas, ImmaParams& p, CUtensorMap& wmap, size_t& smem) {
     using P = ImmaPlan<FMT, FETCH>;
-    auto kernel = gemv_imma_kernel<FMT, FETCH, GROUPS>;
-    ImmaParams p = params_of(a);
-    // One CTA per SM: its sixteen consumer warps share one image of the activations, and whole SMs divide the tiles more
-    // evenly than halves do.
+    p = params_of(a);
     const int tiles = (a.n + kTileRows - 1) / kTileRows;
-    const int grid = tiles < a.sm_count ? tiles : a.sm_count;
-    p.tile_quotient = tiles / grid;
-    p.tile_remainder = tiles % grid;
+    p.tile_quotient = tiles / ctas;
+    p.tile_remainder = tiles % ctas;
     const Ring ring = ring_of(P::kStageBytes, a.members, p.nsb, p.tile_quotient + (p.tile_remainder > 0 ? 1 : 0), a.stages);
     if (ring.stages == 0) return cudaErrorInvalidConfiguration;
     p.stages = ring.stages;
     p.rings = ring.rings;
     p.slots = ring.slots;
-    const size_t smem = imma_fixed_bytes(a.members, p.nsb, p.slots) + static_cast<size_t>(p.stages * p.rings) * P::kStageBytes;
-    static int configured_device = -1;
-    int device = 0;
-    cudaGetDevice(&device);
-    if (configured_device != device) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemLimit));
-        if (e != cudaSuccess) return e;
-        configured_device = device;
-    }
+    smem = imma_fixed_bytes(a.members, p.nsb, p.slots) + static_cast<size_t>(p.stages * p.rings) * P::kStageBytes;
     p.row_bytes = encoded_row_bytes(FMT, a.k);
-    CUtensorMap wmap{};
     if constexpr (FETCH == kBoxes) {
         EncodeTiledFn encode = encode_tiled_fn();
         if (encode == nullptr) return cudaErrorNotSupported;
@@ -973,7 +994,67 @@ cudaError_t launch_groups(const MmaGemvArgs& a) {
     p.accumulate = a.accumulate ? 1 : 0;
     p.n = a.n;
     p.status = a.device_status;
+    return cudaSuccess;
+}
+
+template <typename Kernel>
+cudaError_t allow_shared_memory(Kernel kernel, int& configured_device) {
+    int device = 0;
+    cudaGetDevice(&device);
+    if (configured_device == device) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemLimit));
+    if (e == cudaSuccess) configured_device = device;
+    return e;
+}
+
+template <uint32_t FMT, int FETCH, int GROUPS>
+cudaError_t launch_groups(const MmaGemvArgs& a) {
+    auto kernel = gemv_imma_kernel<FMT, FETCH, GROUPS>;
+    static int configured_device = -1;
+    cudaError_t e = allow_shared_memory(kernel, configured_device);
+    if (e != cudaSuccess) return e;
+    // One CTA per SM: its sixteen consumer warps share one image of the activations, and whole SMs divide the tiles more
+    // evenly than halves do.
+    const int tiles = (a.n + kTileRows - 1) / kTileRows;
+    const int grid = tiles < a.sm_count ? tiles : a.sm_count;
+    ImmaParams p;
+    CUtensorMap wmap{};
+    size_t smem = 0;
+    e = plan<FMT, FETCH>(a, grid, p, wmap, smem);
+    if (e != cudaSuccess) return e;
     return launch_kernel(kernel, dim3(grid), dim3(kThreads), smem, a.stream, wmap, p);
+}
+
+template <uint32_t FMT1, uint32_t FMT2, int GROUPS>
+cudaError_t launch_pair_groups(const MmaGemvArgs& a, const MmaGemvArgs& b) {
+    auto kernel = gemv_imma_pair_kernel<FMT1, FMT2, GROUPS>;
+    static int configured_device = -1;
+    cudaError_t e = allow_shared_memory(kernel, configured_device);
+    if (e != cudaSuccess) return e;
+    // SMs in proportion to the encoded bytes, so that both parts end together
+    const int tiles1 = (a.n + kTileRows - 1) / kTileRows, tiles2 = (b.n + kTileRows - 1) / kTileRows;
+    const double bytes1 = static_cast<double>(tiles1) * block_bytes(FMT1), bytes2 = static_cast<double>(tiles2) * block_bytes(FMT2);
+    int ctas1 = static_cast<int>(a.sm_count * bytes1 / (bytes1 + bytes2) + 0.5);
+    ctas1 = std::max(1, std::min(a.sm_count - 1, ctas1));
+    const int ctas2 = std::min(tiles2, a.sm_count - ctas1);
+    ctas1 = std::min(tiles1, ctas1);
+    ImmaParams p1, p2;
+    CUtensorMap wmap1{}, wmap2{};
+    size_t smem1 = 0, smem2 = 0;
+    e = plan<FMT1, kBoxes>(a, ctas1, p1, wmap1, smem1);
+    if (e == cudaSuccess) e = plan<FMT2, kBoxes>(b, ctas2, p2, wmap2, smem2);
+    if (e != cudaSuccess) return e;
+    return launch_kernel(kernel, dim3(ctas1 + ctas2), dim3(kThreads), std::max(smem1, smem2), a.stream, wmap1, wmap2, p1, p2, ctas1);
+}
+
+template <uint32_t FMT1, uint32_t FMT2>
+cudaError_t launch_pair(const MmaGemvArgs& a, const MmaGemvArgs& b) {
+    switch ((a.members + 1) / 2) {
+        case 1: return launch_pair_groups<FMT1, FMT2, 1>(a, b);
+        case 2: return launch_pair_groups<FMT1, FMT2, 2>(a, b);
+        case 3: return launch_pair_groups<FMT1, FMT2, 3>(a, b);
+        default: return launch_pair_groups<FMT1, FMT2, 4>(a, b);
+    }
 }
 
 template <uint32_t FMT, int FETCH>
@@ -995,6 +1076,15 @@ bool gemv_imma_supports(uint32_t value_type, int k, int n, int members, const vo
     if (members < 1 || members > kMaxMembers || k <= 0 || k % (value_type == kQ8_0 ? 32 : kSuperBlock) != 0 || n < kTileRows) return false;
     if (reinterpret_cast<uintptr_t>(weights) % 16 != 0) return false;
     return ring_of(stage_bytes_of(value_type, fetch_of(value_type, k)), members, superblocks(k), 2, 0).stages != 0;
+}
+
+bool gemv_imma_pairs(const MmaGemvArgs& a, const MmaGemvArgs& b) {
+    return (a.value_type == kQ4_K || a.value_type == kQ5_K) && b.value_type == kQ6_K && fetch_of(kQ6_K, b.k) == kBoxes && a.k == b.k && a.x == b.x &&
+           a.members == b.members && a.members <= kMaxMembers;
+}
+
+cudaError_t launch_gemv_imma_pair(const MmaGemvArgs& a, const MmaGemvArgs& b) {
+    return a.value_type == kQ4_K ? launch_pair<kQ4_K, kQ6_K>(a, b) : launch_pair<kQ5_K, kQ6_K>(a, b);
 }
 
 size_t gemv_imma_image_bytes(int members, int k) { return (image_bytes(members, superblocks(k)) + 255) & ~static_cast<size_t>(255); }

@@ -130,6 +130,9 @@ size_t gemv_imma_image_bytes(int members, int k);
 bool gemv_imma_rotates(uint32_t value_type, int k);   // the image has the element order of Q8_0 blocks fetched in boxes, not the plain one
 cudaError_t launch_gemv_imma_image(const MmaGemvArgs& args, void* image);
 cudaError_t launch_gemv_imma(const MmaGemvArgs& args);
+// Two projections of the same rows in one launch (Q4_K or Q5_K, then Q6_K); one image, if any, for both.
+bool gemv_imma_pairs(const MmaGemvArgs& a, const MmaGemvArgs& b);
+cudaError_t launch_gemv_imma_pair(const MmaGemvArgs& a, const MmaGemvArgs& b);
 
 // tcgen05 GEMV with the weight operand unpacked into tensor memory (qgemv_tmem.cu): Q4_K / Q5_K, up to 8 f32 or
 // 16 bf16 member rows per launch.

@@ -323,8 +323,10 @@ class CudaDenseDecode:
             gemv_fused(self.context, [qk_job, (w.matrices[f"blk.{i}.attn_v"], self.v, False)], self.hidden, self.members,
                        w.vectors[f"blk.{i}.attn_norm"], g.eps, False)
             # one row: every CTA normalises and converts it itself; from two rows on one pre-pass serves the launches,
-            # and only the batch kernel (nine rows and more) writes q and k from one launch
-            self.launches_per_step += 2 if self.members == 1 else (3 if self.members >= 9 else 4)
+            # and only the batch kernel (nine rows and more) writes q and k from one launch; up to eight rows, a Q6_K v
+            # shares the launch of what stands before it
+            paired = self.members <= 8 and self.qk_weights[i].value_type() == Q4_K and w.matrices[f"blk.{i}.attn_v"].value_type() == Q6_K
+            self.launches_per_step += (2 if self.members == 1 else (3 if self.members >= 9 else 4)) - (1 if paired else 0)
         else:
             self._fused([(f"blk.{i}.attn_q", self.q), (f"blk.{i}.attn_k", self.k), (f"blk.{i}.attn_v", self.v)], self.hidden,
                         norm=w.vectors[f"blk.{i}.attn_norm"])

@@ -12,6 +12,7 @@ import pytest
 import torch
 
 import engine_b200
+import engine_b200.decode
 import oracle
 from engine_b200 import synth
 
@@ -493,3 +494,24 @@ def test_narrow_kernel_edges(ctx, gemv_path, vt, n, k, members):
     scale = torch.sqrt(seen.square() @ exact.double().square().T).cpu().numpy()
     # exact weights and 22-bit activations (15-bit ones where eight long rows do not fit the kernel): far inside the bound of the path
     assert np.all(np.abs(y - expected) <= (1e-5 if members * k <= 65536 else 1e-3) * np.maximum(np.abs(expected), scale))
+
+
+# two projections of one normalised input share a launch (Q4_K or Q5_K, then Q6_K): the same bits as one launch each, whatever the
+# split of the SMs -- few and many tiles on either side, ragged ends, rows that convert in the kernel and in a pre-pass
+@pytest.mark.parametrize("first,n1,n2,k", [(12, 5120, 1024, 4096), (13, 16, 4000, 2048), (12, 16000, 17, 2048), (13, 333, 2100, 4096)])
+@pytest.mark.parametrize("members", [1, 2, 4, 8])
+def test_two_projections_in_one_launch(ctx, gemv_path, first, n1, n2, k, members):
+    if gemv_path != 0:
+        pytest.skip("the default path")
+    a = upload(ctx, first, synth.random_weight(first, k, n1, seed=n1), k, n1)
+    b = upload(ctx, 14, synth.random_weight(14, k, n2, seed=n2), k, n2, name="b")
+    rng = np.random.default_rng(members)
+    x = torch.from_numpy(rng.standard_normal((members, k)).astype(np.float32)).to(ctx.device)
+    norm = torch.from_numpy(rng.standard_normal(k).astype(np.float32)).to(ctx.device)
+    ya, yb = torch.empty(members, n1, device=ctx.device), torch.empty(members, n2, device=ctx.device)
+    engine_b200.decode.gemv_fused(ctx, [(a, ya, False), (b, yb, False)], x, members, norm, 1e-6, False)
+    for vt, weight, y in ((first, a, ya), (14, b, yb)):
+        alone = torch.empty_like(y)
+        KERNELS[vt].from_context(ctx).execute_rms_norm(weight, x, norm, 1e-6, alone, members)
+        ctx.synchronize()
+        assert torch.equal(y, alone)
