@@ -128,8 +128,8 @@ void ribn_last_error_detail(const ribn_ctx *ctx, uint64_t *expected, uint64_t *a
  *                   kernel split every weight into two bf16 operands);
  *   "dp4a_prepass": 0 = calls of 1..4 rows on the integer-dot kernel pack their activations inside it, every CTA
  *                   its own copy, instead of in a launch of their own (default 1);
- *   "pdl":          programmatic dependent launch, process-wide: 0 = off, 1 = every kernel of the path, 2 = the GEMV
- *                   kernels and their pre-passes only (default);
+ *   "pdl":          programmatic dependent launch, process-wide: 0 = off, 1 = every kernel of the path, 2 = the
+ *                   projections and their pre-passes, and the layer operators of more than 64 rows (default);
  *   "tc_row_copies": 1 = the f16-tile decode kernel fetches raw weight rows with per-row bulk copies even where one tiled
  *                   TMA box per stage would do (the path of shapes whose rows are not 16-byte aligned);
  *   "tc_ksplit":    split-K factor of the tcgen05 kernels, 0 = choose per shape;
