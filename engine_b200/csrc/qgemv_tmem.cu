@@ -78,6 +78,19 @@ constexpr int kPairs = 4;                  // 64-weight pairs of sub-blocks per 
 constexpr int kPairColumns = 32;           // TMEM columns of one pair: 64 halves per row
 constexpr int kMaxStages = 4;
 
+// A position in a ring, stage and parity of the round: a division per super-block costs its thread a hundred clocks.
+struct RingAt {
+    int stage;
+    uint32_t phase;
+    __device__ __forceinline__ void step(int count, int stages) {
+        stage += count;
+        if (stage >= stages) {
+            stage -= stages;
+            phase ^= 1u;
+        }
+    }
+};
+
 // The hand-overs between workers and issuers poll: a suspended thread wakes some hundred clocks late.  So do waits for memory, except
 // where sixteen worker warps share the SM: there a suspended thread leaves its issue slots to those that unpack.  (A decode
 // step of 32 rows, eight layers: 1474 us with suspended waits, 1404 with polls.)
@@ -537,9 +550,11 @@ __global__ void __launch_bounds__(Roles<NT>::kThreads, NT >= 64 ? 1 : 2) qgemv_t
         // ---------------- one lane streams both rings; the weights do not depend on the kernel before this one ----------------
         if (lane == 0) {
             bool ok = true;
+            RingAt raw_at{0, 0u}, b_at{0, 0u};
             auto issue_raw = [&](int i) {
-                const int s = i % p.raw_stages;
-                if (i >= p.raw_stages && !mbar_wait_bounded_hint(&raw_empty[s], ((i / p.raw_stages) - 1) & 1, kWaitHintNs)) return false;
+                const int s = raw_at.stage;
+                if (i >= p.raw_stages && !mbar_wait_bounded_hint(&raw_empty[s], raw_at.phase ^ 1u, kWaitHintNs)) return false;
+                raw_at.step(1, p.raw_stages);
                 mbar_arrive_expect_tx(&raw_full[s], P::kRawStageBytes);
                 if constexpr (FMT == kQ6_K) {
                     // x in 16-bit elements: the super-block's first byte within the class's rows, rounded down to 16 bytes
@@ -556,8 +571,9 @@ __global__ void __launch_bounds__(Roles<NT>::kThreads, NT >= 64 ? 1 : 2) qgemv_t
                 return true;
             };
             auto issue_b = [&](int i) {
-                const int s = i % p.b_stages;
-                if (i >= p.b_stages && !mbar_wait_bounded_hint(&b_empty[s], ((i / p.b_stages) - 1) & 1, kWaitHintNs)) return false;
+                const int s = b_at.stage;
+                if (i >= p.b_stages && !mbar_wait_bounded_hint(&b_empty[s], b_at.phase ^ 1u, kWaitHintNs)) return false;
+                b_at.step(1, p.b_stages);
                 mbar_arrive_expect_tx(&b_full[s], I::kStageBytes);
                 const uint8_t* src = p.image + static_cast<size_t>(sb_begin + i) * I::kStageBytes;
                 uint8_t* dst = b_ring + static_cast<size_t>(s) * I::kStageBytes;
@@ -590,9 +606,11 @@ __global__ void __launch_bounds__(Roles<NT>::kThreads, NT >= 64 ? 1 : 2) qgemv_t
         const int which = warp == kIssuerWarp ? 0 : 1;
         const uint32_t d_tmem = tmem_base + P::kColD + which * NT;
         bool ok = true;
+        RingAt b_at{0, 0u};
         for (int i = 0; i < local_sb && ok; ++i) {
-            const int bs = i % p.b_stages;
-            ok = __all_sync(0xffffffffu, memory_wait<NT>(&b_full[bs], (i / p.b_stages) & 1));
+            const int bs = b_at.stage;
+            ok = __all_sync(0xffffffffu, memory_wait<NT>(&b_full[bs], b_at.phase));
+            b_at.step(1, p.b_stages);
             if (!ok) break;
             if (i < 4 && which == 0) stamp(p, 1, i * 4);
             const uint64_t desc_b0 = umma_smem_desc_sw128(smem_addr(b_ring + static_cast<size_t>(bs) * I::kStageBytes));
@@ -635,13 +653,15 @@ __global__ void __launch_bounds__(Roles<NT>::kThreads, NT >= 64 ? 1 : 2) qgemv_t
         const uint32_t raw_addr = smem_addr(raw) + static_cast<uint32_t>(row_in_tile) * P::kRowPitch;
         bool ok = true;
 
+        RingAt raw_at{set, 0u};   // raw_stages is at least two, the number of sets
 #pragma unroll 1
         for (int i = set; i < local_sb; i += kSets) {
-            const int s = i % p.raw_stages;
-            if (ok && !memory_wait<NT>(&raw_full[s], (i / p.raw_stages) & 1)) {
+            const int s = raw_at.stage;
+            if (ok && !memory_wait<NT>(&raw_full[s], raw_at.phase)) {
                 atomicExch(p.status, kDeviceWaitTimeout);
                 ok = false;
             }
+            raw_at.step(kSets, p.raw_stages);
             if (i < 4 && quadrant == 0 && set == 0) stamp(p, 2 + half, 2 + i * 4);
             const int abuf = i % AB;
             if constexpr (FMT == kQ6_K) {
