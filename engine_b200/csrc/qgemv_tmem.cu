@@ -456,25 +456,45 @@ __device__ __forceinline__ void unpack_pair(uint32_t quant_addr, uint32_t fifth_
     }
 }
 
-// Q6_K: one group pair of a 128-weight chunk.  `la`, `lb`: the chunk's two runs of 32 low-nibble bytes, `qh` its 32
-// two-bit bytes (all at 2-byte alignment); V0 / V0 + 1 are the groups that go to out_lo / out_hi.  A quant byte
+// Q6_K: the 64 low-nibble bytes and 32 two-bit bytes of a 128-weight chunk, which start WORD words and `shift` bits behind a
+// 16-byte boundary: eight 128-bit loads for both group pairs.
+template <int WORD>
+__device__ __forceinline__ void q6_chunk(uint32_t ql_base, uint32_t qh_base, uint32_t shift, uint32_t (&ql)[16], uint32_t (&qh)[8]) {
+    uint32_t w[20];
+#pragma unroll
+    for (int v = 0; v < 5; ++v) {
+        const uint4 x = lds128(ql_base + 16 * v);
+        w[4 * v] = x.x; w[4 * v + 1] = x.y; w[4 * v + 2] = x.z; w[4 * v + 3] = x.w;
+    }
+#pragma unroll
+    for (int k = 0; k < 16; ++k) ql[k] = __funnelshift_r(w[k + WORD], w[k + WORD + 1], shift);
+#pragma unroll
+    for (int v = 0; v < 3; ++v) {
+        const uint4 x = lds128(qh_base + 16 * v);
+        w[4 * v] = x.x; w[4 * v + 1] = x.y; w[4 * v + 2] = x.z; w[4 * v + 3] = x.w;
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) qh[k] = __funnelshift_r(w[k + WORD], w[k + WORD + 1], shift);
+}
+
+// Q6_K: one group pair of a 128-weight chunk.  `ql`: the chunk's two runs of 32 low-nibble bytes, `qh` its 32
+// two-bit bytes; V0 / V0 + 1 are the groups that go to out_lo / out_hi.  A quant byte
 // (q << 2) under the magic byte is the half 1024 + 4 q; minus 1152 that is 4 (q - 32), exactly; times f16(factor / 4) it is
 // the weight with one rounding relative to its own size (folding the offset into the addend of one HFMA2 would round
 // relative to 4 q, twice as coarse at the centre of the range, and 1152 f is not exact).
 template <int V0>
-__device__ __forceinline__ void unpack_pair_q6(uint32_t la, uint32_t lb, uint32_t qh, const float (&factor)[4], uint32_t (&out_lo)[16],
+__device__ __forceinline__ void unpack_pair_q6(const uint32_t (&ql)[16], const uint32_t (&qh)[8], const float (&factor)[4], uint32_t (&out_lo)[16],
                                                uint32_t (&out_hi)[16]) {
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
-        const uint4 a = lds128_unaligned(la + 16 * half), b = lds128_unaligned(lb + 16 * half), h = lds128_unaligned(qh + 16 * half);
-        const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w}, hw[4] = {h.x, h.y, h.z, h.w};
         const float f0 = factor[half], f1 = factor[2 + half];      // the scale of each run of 16 weights
         const uint32_t mul0 = half2_bits(f0 * 0.25f, f0 * 0.25f);
         const uint32_t mul1 = half2_bits(f1 * 0.25f, f1 * 0.25f);
         constexpr uint32_t kCentre = 0x64806480u;   // 1152 = 1024 + 4 * 32
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const uint32_t b0 = q6_bytes<V0>(aw[i], bw[i], hw[i]), b1 = q6_bytes<V0 + 1>(aw[i], bw[i], hw[i]);
+            const int k = 4 * half + i;
+            const uint32_t b0 = q6_bytes<V0>(ql[k], ql[8 + k], qh[k]), b1 = q6_bytes<V0 + 1>(ql[k], ql[8 + k], qh[k]);
             out_lo[half * 8 + i * 2 + 0] = hmul2(hsub2(__byte_perm(b0, kMagicBytes, 0x4240), kCentre), mul0);   // positions 0, 2
             out_lo[half * 8 + i * 2 + 1] = hmul2(hsub2(__byte_perm(b0, kMagicBytes, 0x4341), kCentre), mul0);   // positions 1, 3
             out_hi[half * 8 + i * 2 + 0] = hmul2(hsub2(__byte_perm(b1, kMagicBytes, 0x4240), kCentre), mul1);
@@ -653,6 +673,8 @@ __global__ void __launch_bounds__(Roles<NT>::kThreads, NT >= 64 ? 1 : 2) qgemv_t
         const uint32_t raw_addr = smem_addr(raw) + static_cast<uint32_t>(row_in_tile) * P::kRowPitch;
         bool ok = true;
 
+        // Q6_K: how far behind a 16-byte boundary the rows of this thread's class start
+        const uint32_t class_start = FMT == kQ6_K ? (static_cast<uint32_t>(row_in_tile / (kRows / p.row_classes)) * p.row_bytes) & 15u : 0u;
         RingAt raw_at{set, 0u};   // raw_stages is at least two, the number of sets
 #pragma unroll 1
         for (int i = set; i < local_sb; i += kSets) {
@@ -665,16 +687,26 @@ __global__ void __launch_bounds__(Roles<NT>::kThreads, NT >= 64 ? 1 : 2) qgemv_t
             if (i < 4 && quadrant == 0 && set == 0) stamp(p, 2 + half, 2 + i * 4);
             const int abuf = i % AB;
             if constexpr (FMT == kQ6_K) {
-                const uint32_t row_class = static_cast<uint32_t>(row_in_tile) / static_cast<uint32_t>(kRows / p.row_classes);
-                const uint32_t blk = raw_addr + static_cast<uint32_t>(s) * P::kRawStageBytes +
-                                     ((((row_class * p.row_bytes) & 15u) + static_cast<uint32_t>(sb_begin + i) * 210u) & 15u);
+                const uint32_t row_start = raw_addr + static_cast<uint32_t>(s) * P::kRawStageBytes;   // on a 16-byte boundary
+                const uint32_t behind = (class_start + static_cast<uint32_t>(sb_begin + i) * 210u) & 15u;
+                const uint32_t blk = row_start + behind;
                 const float d = f16_bits_to_f32(lds_u16(blk + 208));
                 const bool wide = !(fabsf(d) <= 1.0f);   // kept symmetrical with the other formats: beyond it d multiplies afterwards
                 if (!(fabsf(d) < 32.0f)) atomicExch(p.status, kDeviceScaleRange);
                 const uint32_t d2 = half2_bits(d, d);
                 const float fd = wide ? 1.0f : d;
                 // this half's chunk of 128 weights: 64 low-nibble bytes, 32 two-bit bytes, eight int8 scales
-                const uint32_t la = blk + 64 * half, lb = la + 32, qh = blk + 128 + 32 * half, sc = blk + 192 + 8 * half;
+                const uint32_t sc = blk + 192 + 8 * half;
+                uint32_t ql[16], qh[8];
+                {
+                    const uint32_t ql_base = row_start + 64 * half, qh_base = row_start + 128 + 32 * half, shift = (behind & 2u) * 8u;
+                    switch (behind >> 2) {   // the same for the rows of a class
+                        case 0: q6_chunk<0>(ql_base, qh_base, shift, ql, qh); break;
+                        case 1: q6_chunk<1>(ql_base, qh_base, shift, ql, qh); break;
+                        case 2: q6_chunk<2>(ql_base, qh_base, shift, ql, qh); break;
+                        default: q6_chunk<3>(ql_base, qh_base, shift, ql, qh); break;
+                    }
+                }
 #pragma unroll
                 for (int jj = 0; jj < 2; ++jj) {
                     const int j = half * 2 + jj;
@@ -684,8 +716,8 @@ __global__ void __launch_bounds__(Roles<NT>::kThreads, NT >= 64 ? 1 : 2) qgemv_t
 #pragma unroll
                     for (int r = 0; r < 4; ++r) factor[r] = fd * static_cast<float>(lds_s8(sc + 4 * jj + r));
                     uint32_t out_lo[16], out_hi[16];
-                    if (jj == 0) unpack_pair_q6<0>(la, lb, qh, factor, out_lo, out_hi);
-                    else unpack_pair_q6<2>(la, lb, qh, factor, out_lo, out_hi);
+                    if (jj == 0) unpack_pair_q6<0>(ql, qh, factor, out_lo, out_hi);
+                    else unpack_pair_q6<2>(ql, qh, factor, out_lo, out_hi);
                     if (wide) {
 #pragma unroll
                         for (int r = 0; r < 16; ++r) {
