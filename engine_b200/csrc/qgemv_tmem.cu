@@ -422,12 +422,13 @@ __global__ void __launch_bounds__(1024) tmem_image_kernel(const TmemParams p, in
 // A pair is 32 quant bytes: the low nibbles are sub-block 2j (32 weights), the high nibbles sub-block 2j+1.
 // out_lo / out_hi: 16 registers = 32 halves each, K order [e0, e2, e1, e3] within every group of four.
 // mul_a / mul_b: the factor of each sub-block as a half pair; every quant is brought to the low mantissa bits of the
-// half 1024, so that one HFMA2 with -1024 * factor as addend leaves q * factor.
+// half 1024, so that one HFMA2 with -1024 * factor as addend leaves q * factor; the high nibbles stay four bits higher, under the
+// half 64 (64 + q, addend -64 * factor): the same single rounding, and two shifts less per eight weights.
 template <uint32_t FMT>
 __device__ __forceinline__ void unpack_pair(uint32_t quant_addr, uint32_t fifth_addr, int j, uint32_t mul_a, uint32_t mul_b, uint32_t (&out_lo)[16],
                                             uint32_t (&out_hi)[16]) {
     const uint32_t add_a = hmul2(mul_a, 0xe400e400u);    // -1024 * factor
-    const uint32_t add_b = hmul2(mul_b, 0xe400e400u);
+    const uint32_t add_b = hmul2(mul_b, 0xd400d400u);    // -64 * factor
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
         const uint4 q = lds128(quant_addr + 16 * half);
@@ -438,15 +439,16 @@ __device__ __forceinline__ void unpack_pair(uint32_t quant_addr, uint32_t fifth_
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const uint32_t w = qw[i];
-            uint32_t a0 = and_or(w, 0x000f000fu, kMagic), a1 = and_or(w >> 8, 0x000f000fu, kMagic);
-            uint32_t b0 = and_or(w >> 4, 0x000f000fu, kMagic), b1 = and_or(w >> 12, 0x000f000fu, kMagic);
+            const uint32_t upper = w >> 8;
+            uint32_t a0 = and_or(w, 0x000f000fu, kMagic), a1 = and_or(upper, 0x000f000fu, kMagic);
+            uint32_t b0 = and_or(w, 0x00f000f0u, 0x54005400u), b1 = and_or(upper, 0x00f000f0u, 0x54005400u);
             if (FMT == kQ5_K) {
                 // byte p of the fifth-bit bytes carries, in bit s, the fifth bit of position p of sub-block s
                 const uint32_t bits = fw[i] >> (2 * j);
                 a0 = and_or(bits << 4, 0x00100010u, a0);
                 a1 = and_or(bits >> 4, 0x00100010u, a1);
-                b0 = and_or(bits << 3, 0x00100010u, b0);
-                b1 = and_or(bits >> 5, 0x00100010u, b1);
+                b0 = and_or(bits << 7, 0x01000100u, b0);
+                b1 = and_or(bits >> 1, 0x01000100u, b1);
             }
             out_lo[half * 8 + i * 2 + 0] = hfma2(a0, mul_a, add_a);
             out_lo[half * 8 + i * 2 + 1] = hfma2(a1, mul_a, add_a);
