@@ -1,5 +1,5 @@
 // Dequant-fused GEMV for 1..8 activation rows per launch on the integer tensor-core instruction
-// (mma.sync m16n8k32 u8 x s8 for Q4_K and Q5_K, m16n8k16 s8 x s8 for Q6_K; s32 accumulate).
+// (mma.sync m16n8k32 u8 x s8 for Q4_K and Q5_K, s8 x s8 for Q8_0, m16n8k16 s8 x s8 for Q6_K; s32 accumulate).
 //
 //   y[m][n] = sum_k dequant(W[n][k]) * x[m][k]
 //
@@ -24,6 +24,13 @@
 // more (set the top bit, subtract 32 without a borrow between bytes, clear the top bit again), which needs no
 // block sums.  Super-blocks are 210 bytes: every second one starts two bytes off a word boundary, and its words
 // are funnel-shifted out of two aligned loads.
+// Q8_0: the signed instruction; see block_q8.
+// What bounds a call: one row of a few megabytes is start-up (1.6 us from the end of the kernel before to the first multiply:
+// loads, one conversion per warp, instructions fetched for the first time), then issue slots (about 67 weights per clock and
+// SM, HBM delivers 42), then HBM.  So the work is laid out for few barriers and one conversion per SM: one CTA per SM, two groups of
+// eight consumer warps that share the image and take row tiles in turn.  Measured, two CTAs of eight warps per SM before:
+// Q4_K one row 12288 x 4096 9.6 -> 7.8 us; Q8_0 one row 4096 x 4096 10.9 -> 4.5 us and 12288 x 4096 25.8 -> 10.0 us, Q6_K three
+// unaligned rows 1024 x 5120 10.6 -> 6.6 us (both on the integer-dot kernel before).
 // Rounding: the weights are exact; an activation carries 2^-22 of its super-block's largest magnitude, all
 // integer sums are exact, and a row's result does not depend on the rows launched with it.
 //

@@ -22,7 +22,10 @@
 //     call by a pre-pass in exactly the swizzled K-major tiles the MMA reads, and streamed from L2 into a
 //     shared-memory ring with bulk copies next to the weights;
 //   * the accumulator is read back once, at the end of the CTA's K range.
-// About 1.5 thread instructions per weight whatever the number of member rows.
+// What bounds it: issue slots of the unpacking (two CTAs of eight worker warps per SM take 1.1 us per pair of super-blocks of 128
+// rows), and outside the loop the pre-pass and the exchange of K splits, 6 and 7 us of a call.  Measured, before the hand-overs
+// polled and the unpacking shed its repeated loads, shifts and divisions: 16 rows Q4_K 12288 x 4096 19.1 -> 17.9 us, 64 rows Q6_K
+// 4096 x 12288 31.0 -> 28.2 us, 16 rows Q6_K 12288 x 8192 41.1 -> 33.4 us.
 //
 // Q6_K (210-byte super-blocks, no minima): the quant under the magic byte is 1024 + 4 q; minus 1152 it is 4 (q - 32)
 // exactly, and one HMUL2 with f16(d * sc / 4) makes the weight.  A TMA box must start on a 16-byte boundary, so its
