@@ -47,6 +47,7 @@
 #include "internal.h"
 #include "pack_activations.cuh"
 #include "pipeline.cuh"
+#include "row_copy.h"
 #include "tc_host.h"
 #include "tcgen05.cuh"
 #include "unpack.cuh"
@@ -649,19 +650,22 @@ __device__ __forceinline__ void gemv_imma_body(const CUtensorMap& wmap, const Im
                         for (int b = 0; b < boxes; ++b) tma_load_2d(stage + b * P::kBoxBytes, &wmap, x + b * (P::kBoxSpan / 8), row0, bar);
                     }
                 } else {
-                    // lane = (box, row): the row's share of the box from the 16-byte boundary below, up to the one above
+                    // lane = (box, row): the row's share of the box from the 16-byte boundary below, up to the one above, and no
+                    // further than the tensor reaches
                     static_assert(P::kBoxesPerStage * kTileRows <= 32, "one copy per lane");
                     const int row = lane & (kTileRows - 1), b = lane >> 4;
                     const unsigned long long row_start = static_cast<unsigned long long>(row0 + row) * p.row_bytes;
                     const unsigned long long from = row_start + static_cast<unsigned long long>(chunk * P::kBoxesPerStage + b) * P::kBoxSpan;
                     const unsigned long long to = min(from + P::kBoxSpan, row_start + p.row_bytes);
-                    const unsigned long long first = from & ~15ull;
-                    const bool mine = b < boxes && row0 + row < p.n;
-                    const uint32_t bytes = mine ? static_cast<uint32_t>(((to + 15ull) & ~15ull) - first) : 0u;
-                    const uint32_t total = __reduce_add_sync(0xffffffffu, bytes);
+                    RowCopy copy{0ull, 0u, 0u};
+                    if (b < boxes && row0 + row < p.n) copy = row_copy(from, to, p.weight_bytes);
+                    uint8_t* target = stage + b * P::kBoxBytes + row * P::kRowPitch;
+                    for (uint32_t i = 0; i < copy.tail; ++i) target[copy.bytes + i] = p.weights[copy.first + copy.bytes + i];
+                    const uint32_t total = __reduce_add_sync(0xffffffffu, copy.bytes);
+                    __syncwarp();   // the tail is in place before the stage is said to be
                     if (lane == 0) mbar_arrive_expect_tx(bar, total);
                     __syncwarp();
-                    if (mine) bulk_copy_g2s(stage + b * P::kBoxBytes + row * P::kRowPitch, p.weights + first, bytes, bar);
+                    if (copy.bytes > 0) bulk_copy_g2s(target, p.weights + copy.first, copy.bytes, bar);
                 }
             }
             walk.step(stages);
@@ -983,6 +987,7 @@ cudaError_t plan(const MmaGemvArgs& a, int ctas, ImmaParams& p, CUtensorMap& wma
     p.slots = ring.slots;
     smem = imma_fixed_bytes(a.members, p.nsb, p.slots) + static_cast<size_t>(p.stages * p.rings) * P::kStageBytes;
     p.row_bytes = encoded_row_bytes(FMT, a.k);
+    p.weight_bytes = p.row_bytes * static_cast<unsigned long long>(a.n);
     if constexpr (FETCH == kBoxes) {
         EncodeTiledFn encode = encode_tiled_fn();
         if (encode == nullptr) return cudaErrorNotSupported;
