@@ -377,15 +377,37 @@ bool mma_serves(const ribn_ctx* ctx, const ribn_qweight* w, uint64_t k, uint64_t
     return ribn::gemv_mma_supports(w->value_type, static_cast<int>(k), static_cast<int>(n), per_launch, w->data);
 }
 
+// Rows per launch of a call that the integer tensor-core kernel serves in smaller groups: long rows, of which eight images do not
+// fit shared memory, where only the integer-dot kernel is left.  That kernel rounds the rows to 15 bits instead of 22 and would give a
+// row other bits than a launch of fewer rows gives it.  It is also the slower one: Q8_0 4096 x 12288, eight rows, f32: 63.2 us, in
+// two launches of four 37.3; Q6_K 4096 x 11520 68.1 and 45.3, six rows 61.4 and 41.9.  0: not such a call (rows that are too long for
+// the integer-dot kernel as well stay with the f32 kernel, which beats groups of two: Q6_K 5120 x 25600, eight rows, 178 and 246 us).
+uint32_t imma_group(const ribn_ctx* ctx, const ribn_qweight* w, uint64_t k, uint64_t n, uint32_t members) {
+    if (ctx->mma_gemv == 0 || ctx->gemv_path != 0 || ctx->imma_gemv == 0 || mma_serves(ctx, w, k, n, members)) return 0;
+    if (members <= 8 && members > static_cast<uint32_t>(ctx->imma_max_members)) return 0;
+    if (!ribn::gemv_dp4a_fits(w->value_type, static_cast<int>(k), members < 4 ? static_cast<int>(members) : 4)) return 0;
+    uint32_t rows = 8;
+    while (rows > 0 && !ribn::gemv_imma_supports(w->value_type, static_cast<int>(k), static_cast<int>(n), static_cast<int>(rows), w->data)) --rows;
+    return rows < members ? rows : 0;
+}
+
+// Activation images that an earlier projection of a fused call left in the workspace: bit 0 = the f16 image of this x, bit 1 = the
+// int8 image (the two narrow kernels keep different images, side by side), bit 2 = the one of Q8_0; the int8 images are those of
+// launches of `group` rows.
+struct Images {
+    unsigned made = 0;
+    uint32_t group = 8;
+};
+
 // Arguments of the integer tensor-core kernel for rows m0 .. of a call.
 ribn::MmaGemvArgs imma_args(const ribn_ctx* ctx, const ribn_qweight* w, uint64_t k, uint64_t n, const void* x, int x_dtype, int mode,
-                            const float* norm_weight, float eps, void* y, int y_dtype, uint32_t members, bool accumulate, uint32_t m0) {
+                            const float* norm_weight, float eps, void* y, int y_dtype, uint32_t members, bool accumulate, uint32_t m0, uint32_t group = 8) {
     ribn::MmaGemvArgs a{};
     a.weights = static_cast<const uint8_t*>(w->data);
     a.value_type = w->value_type;
     a.k = static_cast<int>(k);
     a.n = static_cast<int>(n);
-    a.members = static_cast<int>(members - m0 < 8 ? members - m0 : 8);
+    a.members = static_cast<int>(members - m0 < group ? members - m0 : group);
     a.x = static_cast<const uint8_t*>(x) + static_cast<uint64_t>(m0) * k * (mode == 2 ? 2 : 1) * dtype_bytes(x_dtype);
     a.x_bf16 = x_dtype == RIBN_BF16;
     a.mode = mode;
@@ -402,12 +424,12 @@ ribn::MmaGemvArgs imma_args(const ribn_ctx* ctx, const ribn_qweight* w, uint64_t
 }
 
 // Where the images of a call of that kernel start in the workspace: behind the ones the f16 kernel would keep for the same call.
-// Q8_0 rows may keep their images in an order of their own, behind the plain ones.
+// Q8_0 rows may keep their images in an order of their own, behind the plain ones (which take no more than one launch per row would).
 uint64_t imma_image_offset(const ribn::MmaGemvArgs& a, uint32_t members) {
     const uint64_t launches = (members + 7) / 8;
     const int per_launch = members < 8 ? static_cast<int>(members) : 8;
     uint64_t offset = launches * ribn::gemv_mma_image_bytes(per_launch, a.k, 2);
-    if (ribn::gemv_imma_rotates(a.value_type, a.k)) offset += launches * ribn::gemv_imma_image_bytes(per_launch, a.k);
+    if (ribn::gemv_imma_rotates(a.value_type, a.k)) offset += members * ribn::gemv_imma_image_bytes(1, a.k);
     return offset;
 }
 
@@ -427,29 +449,32 @@ cudaError_t imma_image(const ribn_ctx* ctx, ribn::MmaGemvArgs& a, bool shared_im
     return ready ? cudaSuccess : ribn::launch_gemv_imma_image(a, image);
 }
 
-// `images_made` (fused calls: shared by the projections of one input): bit 0 = the f16 image of this x is in the
-// workspace, bit 1 = the int8 image is (the two narrow kernels keep different images, side by side), bit 2 = the one of Q8_0.
+// `images`: fused calls, shared by the projections of one input.
 int enqueue_mma(ribn_ctx* ctx, const ribn_qweight* w, uint64_t k, uint64_t n, const void* x, int x_dtype, int mode, const float* norm_weight,
-                float eps, void* y, int y_dtype, uint32_t members, bool accumulate, unsigned* images_made, bool shared_image = false) {
+                float eps, void* y, int y_dtype, uint32_t members, bool accumulate, Images* images, bool shared_image = false) {
     const bool x_bf16 = x_dtype == RIBN_BF16;
     const uint64_t x_row_bytes = k * (mode == 2 ? 2 : 1) * dtype_bytes(x_dtype);
-    unsigned none_made = 0;
-    if (images_made == nullptr) images_made = &none_made;
-    if (imma_serves(ctx, w, k, n, members)) {
+    Images none_made;
+    if (images == nullptr) images = &none_made;
+    uint32_t group = imma_group(ctx, w, k, n, members);
+    if (group != 0 || imma_serves(ctx, w, k, n, members)) {
+        if (group == 0) group = 8;
         const unsigned made = ribn::gemv_imma_rotates(w->value_type, static_cast<int>(k)) ? 4u : 2u;
+        if (images->group != group) images->made &= 1u;   // images of other launches
+        images->group = group;
         uint64_t offset = 0;
-        for (uint32_t m0 = 0; m0 < members; m0 += 8) {
-            ribn::MmaGemvArgs a = imma_args(ctx, w, k, n, x, x_dtype, mode, norm_weight, eps, y, y_dtype, members, accumulate, m0);
+        for (uint32_t m0 = 0; m0 < members; m0 += group) {
+            ribn::MmaGemvArgs a = imma_args(ctx, w, k, n, x, x_dtype, mode, norm_weight, eps, y, y_dtype, members, accumulate, m0, group);
             if (m0 == 0) offset = imma_image_offset(a, members);
-            cudaError_t e = imma_image(ctx, a, shared_image, (*images_made & made) != 0, offset);
+            cudaError_t e = imma_image(ctx, a, shared_image, (images->made & made) != 0, offset);
             if (e != cudaSuccess) return record_cuda(ctx, e, "activation image launch");
             e = ribn::launch_gemv_imma(a);
             if (e != cudaSuccess) return record_cuda(ctx, e, "GEMV launch");
         }
-        *images_made |= made;
+        images->made |= made;
         return RIBN_OK;
     }
-    const bool image_ready = (*images_made & 1u) != 0;
+    const bool image_ready = (images->made & 1u) != 0;
     uint64_t image_offset = 0;
     for (uint32_t m0 = 0; m0 < members; m0 += 8) {
         ribn::MmaGemvArgs a{};
@@ -495,7 +520,7 @@ int enqueue_mma(ribn_ctx* ctx, const ribn_qweight* w, uint64_t k, uint64_t n, co
         const cudaError_t e = ribn::launch_gemv_mma(a);
         if (e != cudaSuccess) return record_cuda(ctx, e, "GEMV launch");
     }
-    if (image_offset != 0) *images_made |= 1u;
+    if (image_offset != 0) images->made |= 1u;
     return RIBN_OK;
 }
 
@@ -527,8 +552,8 @@ int enqueue_gemv(ribn_ctx* ctx, const ribn_qweight* w, uint64_t k, uint64_t n, c
     if (ctx->gemv_path == 0 && (a.x_bf16 || ctx->tc_f32_activations != 0) && tc_batch && ribn::qgemm_tc_supports(a.value_type, a.k) &&
         members * k * 2 + (1u << 20) <= ctx->workspace_bytes)
         return enqueue_tc(ctx, w, k, n, x, x_dtype, y, y_dtype, members, norm_weight, eps);
-    // Up to eight rows per launch (and wider f32 batches, in groups of eight): half2 unpack + mma.sync.
-    if (mma)
+    // Up to eight rows per launch (and wider f32 batches, in groups of eight): mma.sync.
+    if (mma || imma_group(ctx, w, k, n, members) != 0)
         return enqueue_mma(ctx, w, k, n, x, x_dtype, norm_weight != nullptr ? 1 : 0, norm_weight, eps, y, y_dtype, members, false, nullptr);
     // Path 1: integer-dot kernel.  The activations (normalised first when norm_weight is given) are
     // packed once into the context workspace, then consumed four member rows per launch (the
@@ -651,10 +676,12 @@ int enqueue_fused(ribn_ctx* ctx, const ribn_gemv_job* jobs, uint32_t job_count, 
         return RIBN_OK;
     }
     int64_t smallest = INT64_MAX;
-    bool all_mma = true;
+    bool all_mma = true, all_narrow = true;
     for (uint32_t j = 0; j < job_count; ++j) {
         smallest = std::min<int64_t>(smallest, static_cast<int64_t>(jobs[j].weight->encoded_bytes));
-        all_mma = all_mma && mma_serves(ctx, jobs[j].weight, k, ns[j], members);
+        const bool mma = mma_serves(ctx, jobs[j].weight, k, ns[j], members);
+        all_mma = all_mma && mma;
+        all_narrow = all_narrow && (mma || imma_group(ctx, jobs[j].weight, k, ns[j], members) != 0);
     }
     const bool tc_batch = members >= static_cast<uint32_t>(ctx->tc_min_members) ||
                           (!all_mma && (members >= 5 || (members == 4 && smallest >= ctx->tc_four_row_bytes)));
@@ -671,9 +698,9 @@ int enqueue_fused(ribn_ctx* ctx, const ribn_gemv_job* jobs, uint32_t job_count, 
         }
         return RIBN_OK;
     }
-    if (all_mma) {
+    if (all_narrow) {
         const int mode = swiglu ? 2 : (norm_weight != nullptr ? 1 : 0);
-        unsigned images_made = 0;
+        Images images;
         const bool shared_image = job_count > 1 && mode != 0;
         for (uint32_t j = 0; j < job_count; ++j) {
             if (j + 1 < job_count && members <= 8 && imma_serves(ctx, jobs[j].weight, k, ns[j], members) &&
@@ -685,10 +712,12 @@ int enqueue_fused(ribn_ctx* ctx, const ribn_gemv_job* jobs, uint32_t job_count, 
                                                 jobs[j + 1].y_dtype, members, jobs[j + 1].accumulate != 0, 0);
                 if (ribn::gemv_imma_pairs(a, b)) {
                     uint64_t offset = imma_image_offset(a, members);
-                    cudaError_t e = imma_image(ctx, a, shared_image, (images_made & 2u) != 0, offset);
+                    if (images.group != 8) images.made &= 1u;
+                    images.group = 8;
+                    cudaError_t e = imma_image(ctx, a, shared_image, (images.made & 2u) != 0, offset);
                     if (e != cudaSuccess) return record_cuda(ctx, e, "activation image launch");
                     b.image = a.image;
-                    images_made |= 2u;
+                    images.made |= 2u;
                     e = ribn::launch_gemv_imma_pair(a, b);
                     if (e != cudaSuccess) return record_cuda(ctx, e, "GEMV launch");
                     ++j;
@@ -696,7 +725,7 @@ int enqueue_fused(ribn_ctx* ctx, const ribn_gemv_job* jobs, uint32_t job_count, 
                 }
             }
             const int rc = enqueue_mma(ctx, jobs[j].weight, k, ns[j], x, x_dtype, mode, norm_weight, eps, jobs[j].y_device, jobs[j].y_dtype, members,
-                                       jobs[j].accumulate != 0, &images_made, shared_image);
+                                       jobs[j].accumulate != 0, &images, shared_image);
             if (rc != RIBN_OK) return rc;
         }
         return RIBN_OK;
