@@ -20,10 +20,12 @@ extern "C" long long faults(unsigned long long row_bytes, unsigned long long n, 
             if (to > (row + 1) * row_bytes) to = (row + 1) * row_bytes;
             const ribn::RowCopy c = ribn::row_copy(from, to, total);
             const bool inside = c.first + c.bytes <= total && c.first + c.bytes + c.tail <= total;
-            const bool whole = c.first % 16 == 0 && c.bytes % 16 == 0 && c.tail < 16;
+            const bool whole = c.first % 16 == 0 && c.bytes % 16 == 0 && c.tail % 2 == 0 && c.tail < 16;
             const bool covers = c.first <= from && c.first + c.bytes + c.tail >= to;
             const bool fits = c.bytes + c.tail <= pitch;
-            if (!(inside && whole && covers && fits)) ++bad;
+            // rows of all tiles (of 16) but the last are copied up to the next boundary without a look at the tensor's end
+            const bool plain = row >= (n - 1) / 16 * 16 || (c.tail == 0 && c.first + c.bytes == ((to + 15) & ~15ull));
+            if (!(inside && whole && covers && fits && plain)) ++bad;
         }
     }
     return bad;
