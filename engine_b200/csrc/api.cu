@@ -37,6 +37,7 @@ struct ribn_ctx {
     uint64_t workspace_bytes = 0;
     unsigned int* tickets = nullptr;  // split-K tile counters of the tensor-core GEMM, zero between launches
     int tc_ksplit = 0;              // 0 = choose the split-K factor per shape
+    unsigned int exchange_wait_ns = 100000;   // how long the CTAs of a tile wait for one another's partial tiles
     int tc_split_operands = 0;      // 1 = bf16 batches <= 64 use the prefill GEMM kernel instead of the f16 decode kernel
     int tc_trace = 0;               // builds with -DRIBN_TRACE: 1 = kernels record pipeline clock stamps in the workspace tail
     int tc_row_copies = 0;          // 1 = force the per-row bulk-copy variant of the tensor-core kernel
@@ -293,6 +294,7 @@ int enqueue_tc(ribn_ctx* ctx, const ribn_qweight* w, uint64_t k, uint64_t n, con
     t.scratch_bytes = ctx->workspace_bytes;
     t.tickets = ctx->tickets;
     t.ticket_count = kTicketCount;
+    t.patience_ns = ctx->exchange_wait_ns;
     t.force_ksplit = ctx->tc_ksplit;
     t.force_row_copies = ctx->tc_row_copies;
     t.trace = nullptr;
@@ -347,6 +349,7 @@ int enqueue_tmem(ribn_ctx* ctx, const ribn_qweight* w, uint64_t k, uint64_t n, c
     a.scratch_bytes = ctx->workspace_bytes;
     a.tickets = ctx->tickets;
     a.ticket_count = kTicketCount;
+    a.patience_ns = ctx->exchange_wait_ns;
     a.force_ksplit = ctx->tc_ksplit;
     a.stages = ctx->mma_stages;
     a.image_ready = image_ready;
@@ -949,6 +952,10 @@ int ribn_set_option(ribn_ctx* ctx, const char* name, int64_t value) {
     }
     if (std::strcmp(name, "tc_ksplit") == 0 && value >= 0 && value <= 64) {
         ctx->tc_ksplit = static_cast<int>(value);
+        return RIBN_OK;
+    }
+    if (std::strcmp(name, "exchange_wait_ns") == 0 && value >= 0 && value <= 1000000000) {
+        ctx->exchange_wait_ns = static_cast<unsigned int>(value);
         return RIBN_OK;
     }
     if (std::strcmp(name, "tc_split_operands") == 0 && (value == 0 || value == 1)) {

@@ -155,6 +155,7 @@ struct TmemGemvArgs {
     size_t scratch_bytes;
     unsigned int* tickets;    // zero-initialised counters, one per row tile
     int ticket_count;
+    unsigned int patience_ns; // how long CTAs that share a tile wait for one another (split_exchange.cuh), 0 = not at all
     int force_ksplit;         // 0 = choose
     int stages;               // raw ring depth, 0 = as deep as fits
     bool image_ready;         // the activation tiles of this x are in the scratch already (an earlier projection of the same call)
@@ -185,6 +186,7 @@ struct TcArgs {
     size_t scratch_bytes;
     unsigned int* tickets;    // zero-initialised counters, one per output tile
     int ticket_count;
+    unsigned int patience_ns; // how long CTAs that share a tile wait for one another (split_exchange.cuh), 0 = not at all
     int force_ksplit;         // 0 = choose
     long long* trace;         // diagnostics buffer of the decode kernel (see TcParams), or null
     int force_row_copies;     // 1 = per-row bulk copies even where one tiled TMA box per stage would do

@@ -60,6 +60,7 @@
 #include "formats.cuh"
 #include "internal.h"
 #include "row_dequant.cuh"
+#include "split_exchange.cuh"
 #include "tc_host.h"
 #include "tcgen05.cuh"
 #include "unpack.cuh"
@@ -104,7 +105,7 @@ struct GemmParams {
     int n, m, nsb, ksplit, y_bf16;
     int nt, m_tiles, row_pairs, units;   // tokens per unit; units = row_pairs * m_tiles * ksplit, token tile fastest, K range slowest
     int order;               // SumOrder
-    int cooperative;         // every pair of the grid is resident at once: the CTAs of a tile share the sum of its partial tiles
+    unsigned int patience_ns;   // how long the CTAs of a tile wait for one another to share the sum of its partial tiles; 0: the last one adds
     int ticket_stride;       // departures are counted this far behind the arrivals
     int row_classes;         // P above
     unsigned int row_bytes;
@@ -545,8 +546,9 @@ struct Barriers {
     uint64_t half[2][kSlots];            // second CTA: bytes of its half of B
     uint64_t acc_full[2];                // one commit
     uint64_t acc_empty[2];               // first CTA: the dequant warps of both CTAs
+    unsigned int* word;   // of the tile, in split_exchange.cuh
     uint32_t tmem;
-    uint32_t last_flag;
+    uint32_t range;   // tokens whose partial sums this CTA adds: the first, and behind the last << 16
 };
 static_assert(sizeof(Barriers) <= 512, "the plan sets 512 bytes aside");
 
@@ -611,34 +613,27 @@ __device__ __forceinline__ bool store_unit(const GemmParams& p, int u, uint32_t 
     tcgen05_fence_before_sync();
     __syncwarp();
     if (lane == 0) mbar_arrive_first(address_in_first(&bars->acc_empty[buffer]));
-    // Split-K: the partial tiles of a tile are added in slice order.  With the whole grid resident the CTAs of the tile wait for one
-    // another (bounded) and add a share of the tokens each: one CTA alone reads ksplit partial tiles at what a single SM can have in
-    // flight, 24 us for nine of 128 x 256.  Otherwise the CTA that draws the last ticket adds them (a CTA must not wait for one that
-    // may not have started).
+    // Split-K: the partial tiles of a tile are added in slice order, by all CTAs of the tile where the launch expects them to run
+    // at the same time (split_exchange.cuh), else by the last to arrive.
     if (split) {
         const int ksplit = p.ksplit;
-        unsigned int* ticket = p.tickets + w.token_tile * 2 * p.row_pairs + w.row_tile;
         __threadfence();
         named_barrier_sync(2, kDequantWarps * 32);
         if (worker == 0) {
-            const unsigned int drawn = atomicAdd(ticket, 1u);
-            bool go = drawn == static_cast<unsigned int>(ksplit - 1);
-            if (p.cooperative) {
-                unsigned long long start, now;
-                asm volatile("mov.u64 %0, %globaltimer;" : "=l"(start));
-                now = start;
-                while (!(go = *reinterpret_cast<volatile unsigned int*>(ticket) >= static_cast<unsigned int>(ksplit)) && now - start < 1000000000ull)
-                    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
-                ok = ok && go;
-            } else if (go) {
-                *ticket = 0;   // ready for the next launch
-            }
-            bars->last_flag = go ? 1u : 0u;
+            unsigned int* word = p.tickets + w.token_tile * 2 * p.row_pairs + w.row_tile;
+            bars->word = word;
+            // From the first to the last of the CTA's shares: one between them that another CTA adds gets the same bits from both, and
+            // one range costs the loops below (and the dequantisation beside them) no registers.
+            const uint32_t mine = exchange_arrive(word, ksplit, w.k_slice, p.patience_ns);
+            const int shares = exchange_shares(ksplit);
+            const int first = mine == 0 ? 0 : tokens * (__ffs(static_cast<int>(mine)) - 1) / shares;
+            const int last = mine == 0 ? 0 : tokens * (32 - __clz(static_cast<int>(mine))) / shares;
+            bars->range = static_cast<uint32_t>(first) | static_cast<uint32_t>(last) << 16;
         }
         named_barrier_sync(2, kDequantWarps * 32);
-        if (bars->last_flag != 0) {
+        const int t_begin = static_cast<int>(bars->range & 0xffffu), t_end = static_cast<int>(bars->range >> 16);
+        if (t_begin < t_end) {
             __threadfence();
-            const int t_begin = p.cooperative ? tokens * w.k_slice / ksplit : 0, t_end = p.cooperative ? tokens * (w.k_slice + 1) / ksplit : tokens;
             const long long first_row = static_cast<long long>(w.row_tile) * kBM + 4 * lane;
             const float* partial = p.partial + static_cast<size_t>(w.token0) * n + first_row;
             if (first_row < n) {
@@ -691,11 +686,10 @@ __device__ __forceinline__ bool store_unit(const GemmParams& p, int u, uint32_t 
                 }
             }
         }
-        named_barrier_sync(2, kDequantWarps * 32);   // last_flag is free for the next unit
-        // the last CTA of a tile to leave resets both counters: every CTA of the tile has passed its wait by then
-        if (p.cooperative && worker == 0 && atomicAdd(ticket + p.ticket_stride, 1u) == static_cast<unsigned int>(ksplit - 1)) {
-            ticket[p.ticket_stride] = 0;
-            *ticket = 0;
+        named_barrier_sync(2, kDequantWarps * 32);   // `range` is free for the next unit
+        if (p.patience_ns != 0 && worker == 0) {
+            unsigned int* word = bars->word;
+            if (exchange_depart(word + p.ticket_stride) == static_cast<unsigned int>(ksplit - 1)) exchange_reset(word, word + p.ticket_stride);
         }
     }
     return ok;
@@ -1031,7 +1025,8 @@ cudaError_t launch_format(const TcArgs& a) {
     if (image_bytes + factor_bytes > a.scratch_bytes) return cudaErrorMemoryAllocation;
     if (p.ksplit > 1 && (image_bytes + factor_bytes + plane_bytes * p.ksplit > a.scratch_bytes || 2 * p.row_pairs * p.m_tiles > a.ticket_count)) p.ksplit = 1;
     p.units = p.row_pairs * p.m_tiles * p.ksplit;
-    p.cooperative = p.ksplit > 1 && p.units <= pairs && 4 * p.row_pairs * p.m_tiles <= a.ticket_count ? 1 : 0;
+    // one round of units: the CTAs of a tile are likely to run at the same time
+    p.patience_ns = p.ksplit > 1 && p.units <= pairs && 4 * p.row_pairs * p.m_tiles <= a.ticket_count ? a.patience_ns : 0;
     p.ticket_stride = a.ticket_count / 2;
     uint8_t* image = static_cast<uint8_t*>(a.scratch);
     float* factor = reinterpret_cast<float*>(image + image_bytes);

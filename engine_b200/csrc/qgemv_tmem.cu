@@ -38,8 +38,8 @@
 // CTA = 128 rows x a K range; grid = row tiles x K splits.  Warps 0..7 are workers (thread = row; warps 0..3
 // expand the first 128 weights of every super-block, warps 4..7 the second 128), warp 8 streams the raw
 // weights and the activation tiles, warp 9 issues the MMAs and owns the TMEM allocation.  Partial results of
-// K splits meet in global scratch: the CTA that draws the last ticket of a row tile adds them in split order
-// (deterministic).
+// K splits meet in global scratch and are added in split order, by the CTAs of the row tile or the last of them (split_exchange.cuh):
+// deterministic.
 //
 // Every wait on an mbarrier is bounded; a wait that runs out sets the status word and every warp still
 // reaches the teardown that frees TMEM.
@@ -56,6 +56,7 @@
 #include "internal.h"
 #include "pack_activations.cuh"
 #include "pipeline.cuh"
+#include "split_exchange.cuh"
 #include "tc_host.h"
 #include "tcgen05.cuh"
 #include "unpack.cuh"
@@ -127,7 +128,7 @@ struct TmemParams {
     float* partial;             // split-K scratch [ksplit][members][n]
     unsigned int* tickets;      // zero-initialised counters: [row tile] arrivals, [ticket_stride + row tile] departures
     int ticket_stride;
-    int cooperative;            // every CTA of the grid is resident at once: the CTAs of a row tile share the sum of its partial tiles
+    unsigned int patience_ns;   // how long the CTAs of a row tile wait for one another to share the sum of its partial tiles; 0: the last one adds
     int k, n, nsb, members, planes, ksplit, raw_stages, b_stages;
     int row_classes;            // 1, or for Q6_K rows that do not start on 16-byte boundaries 2 / 4 / 8: rows n0 + j * classes + c share class c
     unsigned int row_bytes;
@@ -537,7 +538,7 @@ __global__ void __launch_bounds__(Roles<NT>::kThreads, NT >= 64 ? 1 : 2) qgemv_t
     uint64_t* min_empty = min_full + 2;
     uint64_t* d_full = min_empty + 2;
     uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(d_full + 1);
-    uint32_t* last_flag = tmem_holder + 1;
+    uint32_t* exchange_mask = tmem_holder + 1;
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -860,53 +861,23 @@ __global__ void __launch_bounds__(Roles<NT>::kThreads, NT >= 64 ? 1 : 2) qgemv_t
         tcgen05_fence_before_sync();
         if (quadrant == 0) stamp(p, 2 + half, 23);
         // ---------------- split-K: the partial tiles of a row tile are added in split order ----------------
-        // When the whole grid is resident at once (the launcher knows), every CTA of the row tile waits for the others'
-        // partial tiles (bounded) and adds its own share of the tile: the sum is spread over `ksplit` SMs.  Otherwise the
-        // CTA that draws the last ticket adds the whole tile (a CTA must not wait for one that may not have started).
+        // By all CTAs of the row tile where the launch expects them to run at the same time (split_exchange.cuh), else by the last to
+        // arrive.
         if (split) {
             __threadfence();
             named_barrier_sync(1, kWorkers);
-            unsigned int* ticket = p.tickets + blockIdx.x;
+            unsigned int* word = p.tickets + blockIdx.x;
             unsigned int* departed = p.tickets + p.ticket_stride + blockIdx.x;
-            int first_item = 0, last_item = p.members * (kRows / 4);
-            if (threadIdx.x == 0) {
-                if (p.cooperative) {
-                    atomicAdd(ticket, 1u);
-                    unsigned long long start;
-                    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(start));
-                    bool all = true;
-                    unsigned int spins = 0;
-                    while (*reinterpret_cast<volatile unsigned int*>(ticket) < static_cast<unsigned int>(p.ksplit)) {
-                        if ((++spins & 255u) == 0u) {
-                            unsigned long long now;
-                            asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
-                            if (now - start > 1000000000ull) {
-                                all = false;
-                                break;
-                            }
-                        }
-                    }
-                    if (!all) atomicExch(p.status, kDeviceWaitTimeout);
-                    *last_flag = all ? 1u : 0u;
-                } else {
-                    const unsigned int drawn = atomicAdd(ticket, 1u);
-                    const bool last = drawn == static_cast<unsigned int>(p.ksplit - 1);
-                    if (last) *ticket = 0;   // ready for the next launch
-                    *last_flag = last ? 1u : 0u;
-                }
-            }
+            if (threadIdx.x == 0) *exchange_mask = exchange_arrive(word, p.ksplit, static_cast<int>(blockIdx.y), p.patience_ns);
             named_barrier_sync(1, kWorkers);
-            if (p.cooperative) {
-                const int items = p.members * (kRows / 4);
-                first_item = static_cast<int>(static_cast<long long>(items) * blockIdx.y / p.ksplit);
-                last_item = static_cast<int>(static_cast<long long>(items) * (blockIdx.y + 1) / p.ksplit);
-            }
-            // Every CTA that has seen all partial tiles departs; the last one resets both counters.  Counted here, so that the
-            // answer is back by the time the sum is done.
+            // counted here, so that the answer is back by the time the sum is done
             unsigned int departure = 0;
-            if (p.cooperative && threadIdx.x == 0) departure = atomicAdd(departed, 1u);
-            if (*last_flag != 0) {
-                __threadfence();
+            if (p.patience_ns != 0 && threadIdx.x == 0) departure = exchange_depart(departed);
+            uint32_t mine = *exchange_mask;
+            if (mine != 0) __threadfence();
+            while (mine != 0) {
+                int first_item, last_item;
+                exchange_next(mine, exchange_shares(p.ksplit), p.members * (kRows / 4), first_item, last_item);
                 const size_t plane = static_cast<size_t>(p.members) * p.n;
                 const bool vector = (p.n & 3) == 0;
                 for (int idx = first_item + static_cast<int>(threadIdx.x); idx < last_item; idx += kWorkers) {
@@ -950,10 +921,7 @@ __global__ void __launch_bounds__(Roles<NT>::kThreads, NT >= 64 ? 1 : 2) qgemv_t
                     }
                 }
             }
-            if (p.cooperative && threadIdx.x == 0 && departure == static_cast<unsigned int>(p.ksplit - 1)) {
-                *departed = 0;
-                *ticket = 0;
-            }
+            if (p.patience_ns != 0 && threadIdx.x == 0 && departure == static_cast<unsigned int>(p.ksplit - 1)) exchange_reset(word, departed);
         }
         }   // first worker set
     }
@@ -1017,7 +985,7 @@ cudaError_t launch_format(const TmemGemvArgs& a) {
     if (a.force_ksplit > 0 && a.force_ksplit <= nsb && static_cast<size_t>(a.force_ksplit) * a.members * a.n * sizeof(float) <= partial_bytes &&
         tiles <= a.ticket_count)
         ksplit = a.force_ksplit;
-    const bool cooperative = ksplit > 1 && tiles * ksplit <= resident * a.sm_count && 2 * tiles <= a.ticket_count;
+    const bool resident_at_once = ksplit > 1 && tiles * ksplit <= resident * a.sm_count && 2 * tiles <= a.ticket_count;
     static int configured_device = -1;
     int device = 0;
     cudaGetDevice(&device);
@@ -1063,7 +1031,7 @@ cudaError_t launch_format(const TmemGemvArgs& a) {
     p.partial = partial;
     p.tickets = a.tickets;
     p.ticket_stride = a.ticket_count / 2;
-    p.cooperative = cooperative ? 1 : 0;
+    p.patience_ns = resident_at_once ? a.patience_ns : 0;
     p.k = a.k;
     p.n = a.n;
     p.nsb = nsb;

@@ -133,6 +133,9 @@ void ribn_last_error_detail(const ribn_ctx *ctx, uint64_t *expected, uint64_t *a
  *   "tc_row_copies": 1 = the f16-tile decode kernel fetches raw weight rows with per-row bulk copies even where one tiled
  *                   TMA box per stage would do (the path of shapes whose rows are not 16-byte aligned);
  *   "tc_ksplit":    split-K factor of the tcgen05 kernels, 0 = choose per shape;
+ *   "exchange_wait_ns": how long the CTAs of a split-K tile wait for one another before they leave their share of its sum to
+ *                   the last (default 100000; 0 = nobody waits, the last adds the tile alone).  The wait ends by itself: contexts
+ *                   on other streams may use the GPU at the same time;
  *   "gemv_variant": tile geometry of the f32 kernel, 0 = default, 1..3 = alternatives. */
 int ribn_set_option(ribn_ctx *ctx, const char *name, int64_t value);
 
