@@ -135,6 +135,7 @@ SIGNATURES = {
     "ribn_silu_mul": (ctypes.c_int, [_vp, _vp, _vp, _vp, ctypes.c_uint32, ctypes.c_uint64, ctypes.c_uint64]),
     "ribn_silu_mul_typed": (ctypes.c_int, [_vp, _vp, _vp, _vp, ctypes.c_int, ctypes.c_uint32, ctypes.c_uint64, ctypes.c_uint64]),
     "ribn_residual_add": (ctypes.c_int, [_vp, _vp, _vp, ctypes.c_uint64]),
+    "ribn_residual_add_rows": (ctypes.c_int, [_vp, _vp, _vp, ctypes.c_uint64, ctypes.c_uint64]),
     "ribn_argmax": (ctypes.c_int, [_vp, _vp, ctypes.c_uint32, ctypes.c_uint64, _vp]),
     "ribn_tp_create": (ctypes.c_int, [_vp, ctypes.c_uint32, ctypes.c_uint32, ctypes.c_uint64, _vp, ctypes.POINTER(_vp)]),
     "ribn_tp_destroy": (None, [_vp]),

@@ -1413,13 +1413,19 @@ int ribn_silu_mul_typed(ribn_ctx* ctx, const float* gate_device, const float* up
 }
 
 int ribn_residual_add(ribn_ctx* ctx, float* y_device, const float* x_device, uint64_t length) {
+    return ribn_residual_add_rows(ctx, y_device, x_device, 1, length);
+}
+
+int ribn_residual_add_rows(ribn_ctx* ctx, float* y_device, const float* x_device, uint64_t members, uint64_t length) {
     if (ctx == nullptr) return RIBN_E_INVALID_ARGUMENT;
-    if (length == 0) return record(ctx, fail(RIBN_E_INPUT_LENGTH, "residual_add needs at least one value", 1, 0));
+    uint64_t total = 0;
+    if (mul_overflows(members, length, &total)) return record(ctx, fail(RIBN_E_SHAPE_OVERFLOW, "residual_add shape does not fit CUDA launch arguments"));
+    if (total == 0) return record(ctx, fail(RIBN_E_INPUT_LENGTH, "residual_add needs at least one value", 1, 0));
     DeviceGuard guard(ctx->device);
     Failure f = check_device_pointer(ctx, y_device, "accumulator");
     if (f.status == RIBN_OK) f = check_device_pointer(ctx, x_device, "addend");
     if (f.status != RIBN_OK) return record(ctx, f);
-    const cudaError_t e = ribn::launch_residual_add(y_device, x_device, length, ctx->sm_count, ctx->stream);
+    const cudaError_t e = ribn::launch_residual_add(y_device, x_device, members, total, ctx->sm_count, ctx->stream);
     if (e != cudaSuccess) return record_cuda(ctx, e, "residual_add launch");
     return RIBN_OK;
 }

@@ -247,7 +247,7 @@ size_t attention_scratch_bytes(int members, int q_heads, int splits);
 cudaError_t launch_attention_decode(const LayerAttentionArgs& args, void* out, bool out_bf16, void* scratch, int splits);
 cudaError_t launch_silu_mul(const float* gate, const float* up, void* out, bool out_bf16, uint64_t members, uint64_t length, uint64_t in_stride,
                             int sm_count, cudaStream_t stream);
-cudaError_t launch_residual_add(float* y, const float* x, uint64_t total, int sm_count, cudaStream_t stream);
+cudaError_t launch_residual_add(float* y, const float* x, uint64_t rows, uint64_t total, int sm_count, cudaStream_t stream);
 // `counters`: the context's zero-initialised counters (left zero), for rows that several CTAs share.
 cudaError_t launch_argmax(const float* logits, int members, uint64_t length, uint32_t* out, unsigned int* counters, int counter_count, int sm_count,
                           cudaStream_t stream);

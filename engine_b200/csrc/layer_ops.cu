@@ -868,10 +868,10 @@ cudaError_t launch_silu_mul(const float* gate, const float* up, void* out, bool 
     return cudaSuccess;
 }
 
-cudaError_t launch_residual_add(float* y, const float* x, uint64_t total, int sm_count, cudaStream_t stream) {
+cudaError_t launch_residual_add(float* y, const float* x, uint64_t rows, uint64_t total, int sm_count, cudaStream_t stream) {
     unsigned long long blocks = (total / 4 + 255) / 256;
     if (blocks > static_cast<unsigned long long>(sm_count) * 8) blocks = static_cast<unsigned long long>(sm_count) * 8;
-    return launch_kernel_if(dependent_launch(total / 4096), residual_add_kernel, dim3(static_cast<unsigned>(blocks ? blocks : 1)), dim3(256), 0, stream, y, x,
+    return launch_kernel_if(dependent_launch(rows), residual_add_kernel, dim3(static_cast<unsigned>(blocks ? blocks : 1)), dim3(256), 0, stream, y, x,
                          static_cast<unsigned long long>(total));
 }
 

@@ -79,7 +79,9 @@ class CudaDenseOps:
                                                          length, input_row_stride))
 
     def residual_add(self, accumulator: torch.Tensor, addend: torch.Tensor) -> None:
-        self.context.check(self._lib.ribn_residual_add(self.context.handle, accumulator.data_ptr(), addend.data_ptr(), accumulator.numel()))
+        members = accumulator.shape[0] if accumulator.dim() > 1 else 1
+        self.context.check(self._lib.ribn_residual_add_rows(self.context.handle, accumulator.data_ptr(), addend.data_ptr(), members,
+                                                            accumulator.numel() // max(members, 1)))
 
     def argmax(self, logits: torch.Tensor, members: int, output: torch.Tensor) -> None:
         self.context.check(self._lib.ribn_argmax(self.context.handle, logits.data_ptr(), members, logits.numel() // members, output.data_ptr()))

@@ -472,6 +472,9 @@ int ribn_silu_mul_typed(ribn_ctx* ctx, const float* gate_device, const float* up
 
 /* residual_add (model_ops.rs:600-610): y[i] += x[i]. */
 int ribn_residual_add(ribn_ctx* ctx, float* y_device, const float* x_device, uint64_t length);
+/* The same over [members][length] values: with the rows known, those of a prompt chunk (more than 64) start as a dependent
+ * launch, which a decode step's must not (option "pdl"). */
+int ribn_residual_add_rows(ribn_ctx* ctx, float* y_device, const float* x_device, uint64_t members, uint64_t length);
 
 /* argmax / argmax_batch (model_ops.rs:201-314): index of the largest logit per member; NaN never wins,
  * ties go to the lowest index. */
