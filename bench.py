@@ -757,10 +757,6 @@ def main() -> None:
     # One batch size at a time through every matrix, the way a decode step meets them.
     cases = [(vt, n, k, m) for m in MEMBERS for vt in FORMATS for n, k in SHAPES]
     step_bytes = sum(case_bytes(*c) for c in cases)
-    # Launches per call: one for up to two member rows over at most 24 super-blocks (the kernel converts its activations
-    # itself), otherwise an activation pre-pass and the GEMV kernel.
-    launches_per_step = sum(1 if m * (k // 256) <= 40 else 2 for _, _, k, m in cases)
-
     def launch(vt, n, k, m):
         ring = rings[(vt, n, k)]
         weight = ring[cursor[(vt, n, k)] % len(ring)]
@@ -791,7 +787,9 @@ def main() -> None:
             return None
 
     torch.cuda.synchronize()
+    launches_before = ctx._lib.ribn_launches()
     step()  # first launches set per-kernel attributes, which must not happen inside a capture
+    launches_per_step = ctx._lib.ribn_launches() - launches_before   # the projections and their activation pre-passes
     torch.cuda.synchronize()
     step_graph = capture(step)
 

@@ -921,6 +921,8 @@ int ribn_selftest_bounded_wait(ribn_ctx* ctx, uint32_t polls) {
     return RIBN_OK;
 }
 
+uint64_t ribn_launches(void) { return ribn::launch_count(); }
+
 const char* ribn_status_string(int status) {
     switch (status) {
         case RIBN_OK: return "ok";

@@ -55,8 +55,7 @@ cudaError_t launch(const uint8_t* w, uint64_t k, uint64_t n, float* out, int sm_
     const unsigned long long cap = static_cast<unsigned long long>(sm_count) * 8;
     if (blocks > cap) blocks = cap;
     if (blocks == 0) blocks = 1;
-    dequantize_kernel<FMT><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(w, out, k, n, row_bytes, nsb);
-    return cudaGetLastError();
+    return launch_kernel_if(false, dequantize_kernel<FMT>, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, stream, w, out, k, n, row_bytes, nsb);
 }
 
 }  // namespace

@@ -16,6 +16,12 @@ inline int& pdl_switch() {
     return enabled;
 }
 
+// Kernels the calling thread has launched (ribn_launches): every launch of the library goes through launch_kernel_if.
+inline uint64_t& launch_count() {
+    static thread_local uint64_t count = 0;
+    return count;
+}
+
 // pdl_switch(): 0 = off, 1 = every kernel of the path, 2 = the GEMV kernels and their pre-passes only (default;
 // measured on the decode loop: 233 tok/s off, 266 with every kernel, 274 with the GEMV kernels only -- the small
 // layer operators gain nothing from starting early and hold SM slots while they wait).
@@ -32,7 +38,9 @@ cudaError_t launch_kernel_if(bool dependent, void (*kernel)(KernelArgs...), dim3
     attribute[0].val.programmaticStreamSerializationAllowed = 1;
     config.attrs = attribute;
     config.numAttrs = dependent ? 1 : 0;
-    return cudaLaunchKernelEx(&config, kernel, static_cast<KernelArgs>(args)...);
+    const cudaError_t e = cudaLaunchKernelEx(&config, kernel, static_cast<KernelArgs>(args)...);
+    if (e == cudaSuccess) ++launch_count();
+    return e;
 }
 
 template <typename... KernelArgs, typename... Args>

@@ -121,19 +121,18 @@ __global__ void __launch_bounds__(kNormThreads) rms_norm_kernel(const XT* __rest
 cudaError_t launch_rms_norm(const void* x, bool x_bf16, const float* weight, void* y, bool y_bf16, int members,
                             int length, float eps, cudaStream_t stream) {
     const int vecs = (length % 4 == 0) ? length / 4 : 0;
+    const dim3 grid(members), block(kNormThreads);
     if (x_bf16 && y_bf16)
-        rms_norm_kernel<__nv_bfloat16, __nv_bfloat16><<<members, kNormThreads, 0, stream>>>(
-            static_cast<const __nv_bfloat16*>(x), weight, static_cast<__nv_bfloat16*>(y), length, vecs, eps);
-    else if (x_bf16)
-        rms_norm_kernel<__nv_bfloat16, float><<<members, kNormThreads, 0, stream>>>(
-            static_cast<const __nv_bfloat16*>(x), weight, static_cast<float*>(y), length, vecs, eps);
-    else if (y_bf16)
-        rms_norm_kernel<float, __nv_bfloat16><<<members, kNormThreads, 0, stream>>>(
-            static_cast<const float*>(x), weight, static_cast<__nv_bfloat16*>(y), length, vecs, eps);
-    else
-        rms_norm_kernel<float, float><<<members, kNormThreads, 0, stream>>>(static_cast<const float*>(x), weight,
-                                                                              static_cast<float*>(y), length, vecs, eps);
-    return cudaGetLastError();
+        return launch_kernel_if(false, rms_norm_kernel<__nv_bfloat16, __nv_bfloat16>, grid, block, 0, stream, static_cast<const __nv_bfloat16*>(x), weight,
+                                static_cast<__nv_bfloat16*>(y), length, vecs, eps);
+    if (x_bf16)
+        return launch_kernel_if(false, rms_norm_kernel<__nv_bfloat16, float>, grid, block, 0, stream, static_cast<const __nv_bfloat16*>(x), weight,
+                                static_cast<float*>(y), length, vecs, eps);
+    if (y_bf16)
+        return launch_kernel_if(false, rms_norm_kernel<float, __nv_bfloat16>, grid, block, 0, stream, static_cast<const float*>(x), weight,
+                                static_cast<__nv_bfloat16*>(y), length, vecs, eps);
+    return launch_kernel_if(false, rms_norm_kernel<float, float>, grid, block, 0, stream, static_cast<const float*>(x), weight, static_cast<float*>(y),
+                            length, vecs, eps);
 }
 
 namespace {
@@ -150,8 +149,7 @@ __global__ void bounded_wait_selftest_kernel(int* status, uint32_t polls) {
 }  // namespace
 
 cudaError_t launch_bounded_wait_selftest(int* status, uint32_t polls, cudaStream_t stream) {
-    bounded_wait_selftest_kernel<<<1, 32, 0, stream>>>(status, polls);
-    return cudaGetLastError();
+    return launch_kernel_if(false, bounded_wait_selftest_kernel, dim3(1), dim3(32), 0, stream, status, polls);
 }
 
 }  // namespace ribn

@@ -293,6 +293,7 @@ class CudaDenseDecode:
         self.prefill_scratch: dict | None = None
         self.graph = None
         self.launches_per_step = 0
+        self.collectives = 0
         if members > 4:
             # Batches go to the tensor-core kernel, which rounds the f32 activations to f16 (inside the 2e-3 bound).
             context.set_option("tc_f32_activations", 1)
@@ -301,21 +302,15 @@ class CudaDenseDecode:
     def _fused(self, names_outputs, x: torch.Tensor, norm: torch.Tensor | None = None, swiglu: bool = False, accumulate: bool = False) -> None:
         jobs = [(self.weights.matrices[name], y, accumulate) for name, y in names_outputs]
         gemv_fused(self.context, jobs, x, self.members, norm, self.geometry.eps, swiglu)
-        # one launch per projection, plus the activation pre-pass where one runs (from three members on, for wide
-        # two-member inputs, for gated inputs, and whenever several projections share a normalised input)
-        shared = len(jobs) > 1 and norm is not None and self.members >= 2
-        prepass = self.members >= 3 or shared or swiglu or x.shape[-1] // 256 > 24
-        self.launches_per_step += len(jobs) + (1 if prepass else 0)
 
     def _all_reduce(self, t: torch.Tensor) -> None:
         if not self.skip_exchange:
             torch.distributed.all_reduce(t, group=self.group)
-            self.launches_per_step += 1
+            self.collectives += 1
 
     def _exchange(self, slot: int) -> None:
         if not self.skip_exchange:
             self.link.allreduce_residual(slot, self.hidden, self.members, self.geometry.hidden, self.partial_dtype)
-            self.launches_per_step += 1
 
     def _layer(self, i: int) -> None:
         g, s, w = self.geometry, self.shapes, self.weights
@@ -324,11 +319,6 @@ class CudaDenseDecode:
             qk_job = (self.qk_weights[i], self.qk, False) if self.members == 1 else (self.qk_weights[i], self.q, False, self.k)
             gemv_fused(self.context, [qk_job, (w.matrices[f"blk.{i}.attn_v"], self.v, False)], self.hidden, self.members,
                        w.vectors[f"blk.{i}.attn_norm"], g.eps, False)
-            # one row: every CTA normalises and converts it itself; from two rows on one pre-pass serves the launches,
-            # and only the batch kernel (nine rows and more) writes q and k from one launch; up to eight rows, a Q6_K v
-            # shares the launch of what stands before it
-            paired = self.members <= 8 and self.qk_weights[i].value_type() == Q4_K and w.matrices[f"blk.{i}.attn_v"].value_type() == Q6_K
-            self.launches_per_step += (2 if self.members == 1 else (3 if self.members >= 9 else 4)) - (1 if paired else 0)
         else:
             self._fused([(f"blk.{i}.attn_q", self.q), (f"blk.{i}.attn_k", self.k), (f"blk.{i}.attn_v", self.v)], self.hidden,
                         norm=w.vectors[f"blk.{i}.attn_norm"])
@@ -337,7 +327,6 @@ class CudaDenseDecode:
                                          self.max_context, self.active_context)
         self.ops.qk_norm_rope_append(attention, self.q, self.k, self.v)
         self.ops.attention_decode(attention, self.q, self.attended)
-        self.launches_per_step += 3   # head norm + rope + cache append; split-KV attention; merge of the splits
         if parallel and self.link is not None:
             # partial sums of the column-split projection go straight into the link's slot; one kernel pulls the peers'
             self._fused([(f"blk.{i}.attn_output", self.link.partial(0, self.members, g.hidden, self.partial_dtype))], self.attended)
@@ -347,7 +336,6 @@ class CudaDenseDecode:
             self._fused([(f"blk.{i}.attn_output", self.projected)], self.attended)
             self._all_reduce(self.projected)
             self.ops.residual_add(self.hidden, self.projected)
-            self.launches_per_step += 1
         else:
             self._fused([(f"blk.{i}.attn_output", self.hidden)], self.attended, accumulate=True)      # hidden += W attended
         self._fused([(f"blk.{i}.ffn_gate_up", self.gate_up)], self.hidden, norm=w.vectors[f"blk.{i}.ffn_norm"])
@@ -358,20 +346,25 @@ class CudaDenseDecode:
             self._fused([(f"blk.{i}.ffn_down", self.projected)], self.gate_up, swiglu=True)
             self._all_reduce(self.projected)
             self.ops.residual_add(self.hidden, self.projected)
-            self.launches_per_step += 1
         else:
             self._fused([(f"blk.{i}.ffn_down", self.hidden)], self.gate_up, swiglu=True, accumulate=True)
 
     def _forward(self) -> None:
-        self.launches_per_step = 0
         self.ops.embedding(self.weights.matrices["token_embd"], self.tokens, self.hidden)
         for i in range(self.geometry.layers):
             self._layer(i)
         self._fused([("output", self.logits)], self.hidden, norm=self.weights.vectors["output_norm"])
-        self.launches_per_step += 1
         if self.world == 1:
             self.ops.argmax(self.logits, self.members, self.next_tokens)
-            self.launches_per_step += 1
+
+    def _step(self) -> None:
+        """One token per sequence; launches_per_step: this library's kernels and the sums over the ranks."""
+        lib = self.context._lib
+        before, self.collectives = lib.ribn_launches(), 0
+        self._forward()
+        if self.world > 1:
+            self._select_tokens_tensor_parallel()
+        self.launches_per_step = lib.ribn_launches() - before + self.collectives
 
     def _select_tokens_tensor_parallel(self, logits: torch.Tensor | None = None, out: torch.Tensor | None = None) -> None:
         """Each rank holds a slice of the logits: local argmax, then the best (value, index) over the ranks."""
@@ -380,7 +373,6 @@ class CudaDenseDecode:
         rows = logits.shape[0]
         if self.link is not None and out.data_ptr() % 16 == 0 and logits.data_ptr() % 16 == 0:
             self.link.select_tokens(logits, rows, self.shapes["vocab_begin"], out)
-            self.launches_per_step += 1
             return
         local = torch.empty(rows, dtype=torch.int32, device=self.context.device)
         self.ops.argmax(logits, rows, local)
@@ -485,9 +477,7 @@ class CudaDenseDecode:
     def run_step(self) -> None:
         """tokens, positions -> next_tokens (all device resident); appends to the KV cache at `positions`."""
         with torch.cuda.stream(self.context.stream):
-            self._forward()
-            if self.world > 1:
-                self._select_tokens_tensor_parallel()
+            self._step()
 
     def capture(self, advance: bool = False) -> None:
         """Record run_step into a CUDA graph (positions and tokens are read from device memory at replay).
@@ -497,9 +487,7 @@ class CudaDenseDecode:
         torch.cuda.synchronize()
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(graph, stream=self.context.stream):
-            self._forward()
-            if self.world > 1:
-                self._select_tokens_tensor_parallel()
+            self._step()
             if advance:
                 self.tokens.copy_(self.next_tokens)
                 self.positions.add_(1)

@@ -96,6 +96,10 @@ int ribn_synchronize(ribn_ctx *ctx);
  * Nothing is left waiting on the GPU. */
 int ribn_selftest_bounded_wait(ribn_ctx *ctx, uint32_t polls);
 
+/* Kernels that the calling thread has launched through this library so far (the two ends of a call or a captured step tell what it
+ * consists of).  No counterpart in the reference. */
+uint64_t ribn_launches(void);
+
 const char *ribn_status_string(int status);
 /* Message of the last failing call on `ctx`, worded like the Display impl of
  * the reference error (quantized.rs:102-137).  Valid until the next call. */

@@ -64,3 +64,28 @@ def test_residual_add_of_a_decode_step_is_a_plain_launch(own, rows, length, depe
         graph.replay()
     own.synchronize()
     assert torch.equal(y, before + 2)
+
+
+def kernel_nodes(graph):
+    raw, count = ctypes.c_void_p(graph.raw_cuda_graph()), ctypes.c_size_t(4096)
+    nodes, kind = (ctypes.c_void_p * 4096)(), ctypes.c_int()
+    assert runtime().cudaGraphGetNodes(raw, nodes, ctypes.byref(count)) == 0
+    found = 0
+    for i in range(count.value):
+        assert runtime().cudaGraphNodeGetType(ctypes.c_void_p(nodes[i]), ctypes.byref(kind)) == 0
+        found += kind.value == KERNEL_NODE
+    return found
+
+
+# one row, shared images, paired and separate launches, the batch kernel; both geometries' row lengths
+@pytest.mark.parametrize("members", [1, 2, 3, 8, 9, 33])
+@pytest.mark.parametrize("hidden,intermediate", [(4096, 12288), (5120, 6400)])
+def test_launches_per_step_are_the_kernels_of_the_step(own, members, hidden, intermediate):
+    geometry = decode.DenseGeometry(hidden, 2, 16, 4, 128, intermediate, 2048)
+    weights = decode.random_weights(own, geometry, seed=3)
+    decoder = decode.CudaDenseDecode(own, geometry, weights, members, 64)
+    try:
+        graph = captured(own.stream, decoder._step)
+        assert decoder.launches_per_step == kernel_nodes(graph)
+    finally:
+        own.set_option("tc_f32_activations", 0)
