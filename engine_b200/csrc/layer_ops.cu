@@ -877,6 +877,7 @@ cudaError_t launch_residual_add(float* y, const float* x, uint64_t rows, uint64_
 
 cudaError_t launch_argmax(const float* logits, int members, uint64_t length, uint32_t* out, unsigned int* counters, int counter_count, int sm_count,
                           cudaStream_t stream) {
+    if (members <= 0) return cudaErrorInvalidValue;
     // As many CTAs as the rows have pieces of 4096 values, at most four per SM over all rows; one per row where the counters
     // do not reach.
     const uint64_t pieces = (length + kArgmaxThreads * kArgmaxPerThread - 1) / (kArgmaxThreads * kArgmaxPerThread);
@@ -884,7 +885,6 @@ cudaError_t launch_argmax(const float* logits, int members, uint64_t length, uin
     if (parts > pieces) parts = pieces;
     if (static_cast<int64_t>(members) * kArgmaxWordsPerMember > counter_count) parts = 1;
     // members is the grid's y dimension
-    if (members <= 0) return cudaErrorInvalidValue;
     for (int first = 0; first < members; first += 65535) {
         const int rows = members - first < 65535 ? members - first : 65535;
         const cudaError_t e = launch_kernel_if(pdl_switch() == 1, argmax_kernel, dim3(static_cast<unsigned>(parts), rows), dim3(kArgmaxThreads), 0, stream,

@@ -161,7 +161,6 @@ struct Ring {
     }
 };
 // TMEM: accumulators, then (A ring in TMEM) the A ring.  Two buffers of accumulators where tokens leave room, one otherwise.
-template <bool SMEM_A>
 __device__ __forceinline__ int acc_buffers(int nt) { return nt <= kMaxTokens / 2 ? 2 : 1; }
 template <bool SMEM_A>
 __device__ __forceinline__ uint32_t acc_column(int nt, int buffer, int sum) {
@@ -720,7 +719,7 @@ __device__ __forceinline__ bool dequant_warps(const GemmParams& p, uint32_t raw,
                                    : tmem_base + (static_cast<uint32_t>(row_in_tile & ~31) << 16) + kARing + kARingColumns * set + 64 * half;
     const uint32_t raw_full = smem_addr(bars->raw_full), raw_empty = smem_addr(bars->raw_empty), empty = smem_addr(&bars->empty[set][2 * half]);
     const uint32_t full = address_in_first(&bars->full[set][2 * half]);
-    const int buffers = acc_buffers<SMEM_A>(p.nt);
+    const int buffers = acc_buffers(p.nt);
     const int stride = gridDim.x >> 1;
     Ring acc;
     // Super-block b of this CTA's sequence of units lies in raw stage b % kRawStages and belongs to set b % 2.  After a wait that ran out
@@ -893,7 +892,7 @@ qgemm_tc_kernel(const __grid_constant__ RawMaps wmaps, const __grid_constant__ G
             const uint64_t desc_b = umma_smem_desc_sw128(smem_addr(b_tiles));
             const uint64_t desc_a = umma_smem_desc_sw128(smem_addr(a_tiles));
             const uint32_t full = smem_addr(&bars->full[0][0]), empty = smem_addr(&bars->empty[0][0]);
-            const int buffers = acc_buffers<SMEM_A>(p.nt);
+            const int buffers = acc_buffers(p.nt);
             uint32_t polls = kPolls;
             Ring acc;
             uint32_t blocks = 0, stage = 0;
