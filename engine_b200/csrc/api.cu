@@ -438,9 +438,12 @@ uint64_t imma_image_offset(const ribn::MmaGemvArgs& a, uint32_t members) {
 
 // Gives `a` its image when the call is to have one, made now unless `ready`.
 cudaError_t imma_image(const ribn_ctx* ctx, ribn::MmaGemvArgs& a, bool shared_image, bool ready, uint64_t& offset) {
-    // Every CTA converts the activations itself while that is at most about two slices per warp (measured, 3 x 2048: 7.5 -> 5.0
-    // us without the pre-pass, 3 x 4096 and 2 x 8192 slower); several projections of one normalised or gated input of two rows or
-    // more share the image, and silu(gate) * up is worth making once.
+    // Every CTA converts the activations itself while that is at most about two slices per warp; several projections of one
+    // normalised or gated input of two rows or more share the image, and silu(gate) * up is worth making once.  The line at 40 slices
+    // weighs two uses.  Eager calls pay the second launch on the host (inside the kernel and with the pre-pass: Q4_K 4096 rows, 2 x 4096
+    // 5.6 and 6.8 us, 4 x 2560 6.5 and 6.5; Q6_K 1024 rows, 3 x 2048 4.5 and 6.5, 2 x 5120 6.5 and 6.4).  In a captured step the
+    // pre-pass pays from about 24 slices on where there are two rows or more (the same calls 5.4 and 5.0, 6.3 and 5.3, 4.2 and 4.1, 6.1
+    // and 5.2; above the line Q4_K 4 x 4096 7.9 and 6.0, 8 x 2048 7.7 and 5.7).
     const bool by_size = static_cast<uint64_t>(a.members) * ((a.k + 255) / 256) > 40;
     const bool wide = ctx->mma_image_members > 8 ? false
                       : (ctx->mma_image_members == 3 ? by_size : a.members >= ctx->mma_image_members) || (shared_image && a.members >= 2) || a.mode == 2;

@@ -752,8 +752,8 @@ __global__ void __launch_bounds__(kArgmaxThreads) argmax_kernel(const float* __r
 
 // Whether an operator over `rows` rows is launched as a dependent of the kernel before it.  A decode step's operators are not (unless
 // option "pdl" is 1): resident early, they keep the SMs from the projection behind them, whose weights could already be on their
-// way (a step of one row: 2080 us without, 2163 with).  A prompt chunk's kernels are long and fill the SMs, and the launch between
-// them is what a dependent start hides (1987 tokens, four layers: 6640 us without, 6530 with).
+// way (a step of one row: 1910 us without, 2020 with; 32 rows 1374 and 1385).  A prompt chunk's kernels are long and fill the SMs,
+// and the launch between them is what a dependent start hides (1987 tokens, four layers: 6645 us without, 6540 with).
 static bool dependent_launch(uint64_t rows) { return pdl_switch() == 1 || (pdl_switch() == 2 && rows > 64); }
 
 cudaError_t launch_embedding(const uint8_t* weights, uint32_t value_type, int k, unsigned int vocabulary, const uint32_t* tokens,
@@ -779,8 +779,11 @@ cudaError_t launch_qk_norm_rope_append(const LayerAttentionArgs& a) {
 }
 
 // Consecutive tokens of one sequence go to the chunk kernel once the token-by-token walk has enough CTAs to leave the context
-// unsplit (four per SM) and the chunk's row tiles occupy at least half of the SMs; below that the walk, spread over the SMs, is
-// the faster one.
+// unsplit (four per SM) and the chunk's row tiles occupy at least half of the SMs.  Above the first line both give the same bits;
+// below it the walk merges splits, which rounds differently.  The line is not where the times cross, which is earlier: 8 key/value
+// heads of four query heads, behind 512 tokens, walk and chunk: 32 tokens 22.0 and 26.4 us, 64 tokens 36.1 and 26.7, 96 tokens 48.9 and
+// 27.9 (the walk is taken), 112 tokens 58.4 and 28.1, 512 tokens 270 and 91.9 (the chunk is).  The second line is where a shard's
+// two heads are: 128 tokens 27.0 and 28.1, 173 tokens 34.2 and 29.7, 512 tokens 85.5 and 55.5.
 static bool attention_is_chunk(const LayerAttentionArgs& a, int sm_count) {
     const long long tiles = (static_cast<long long>(a.members) * (a.q_heads / a.kv_heads) + kChunkRows - 1) / kChunkRows;
     return a.shared_cache && static_cast<long long>(a.members) * a.kv_heads > 4ll * sm_count && 2 * tiles * a.kv_heads >= sm_count;

@@ -998,7 +998,9 @@ cudaError_t launch_format(const TcArgs& a) {
     const int n_tiles = (a.n + kBM - 1) / kBM;
     p.row_pairs = (n_tiles + 1) / 2;
     // Sums and K ranges follow from the sizes of the call alone.  Up to 128 tokens: even and odd steps; up to 256, and where wide
-    // tiles of 512 would leave more than a fifth of the SMs idle: every third; else one sum.
+    // tiles of 512 would leave more than a fifth of the SMs idle: every third; else one sum.  Nothing in this kernel asks for two
+    // sums; they are the order of additions of the form it replaced, kept so that results keep their bits, and they cost it the plan
+    // with A in tensor memory.
     const long long wide_tiles = static_cast<long long>(n_tiles) * ((a.m + 511) / 512);
     const bool wide = FMT != kQ8_0 && a.m > 256 && wide_tiles * 5 >= static_cast<long long>(a.sm_count) * 4;
     p.order = a.m <= 128 ? kEvenOdd : wide ? kOneSum : kEveryThird;
@@ -1011,8 +1013,11 @@ cudaError_t launch_format(const TcArgs& a) {
     const size_t factor_bytes = (static_cast<size_t>(a.m) * sizeof(float) + 255) & ~static_cast<size_t>(255);
     const size_t partial_space = a.scratch_bytes > x_bytes + factor_bytes ? a.scratch_bytes - x_bytes - factor_bytes : 0;
     p.ksplit = choose_ksplit(tiles, p.nsb, a.sm_count, plane_bytes, partial_space, a.ticket_count);
-    // Hundreds of tokens: a partial tile is megabytes, written and read once more per split (192 tiles of 512 tokens: 127 us
-    // unsplit, 160 us split in two).  K is split then only where the tiles leave more than half of the SMs idle.
+    // Hundreds of tokens: a partial tile is megabytes, written and read once more per split.  K is split then only where the tiles
+    // leave more than half of the SMs idle.  Measured, unsplit and in two: Q4_K 12288 x 4096, 512 tokens 58.0 and 70.7 us; 5120 x 5120,
+    // 512 tokens 38.5 and 50.3; 8192 x 4096, 300 tokens 32.4 and 44.7; Q6_K 4096 x 12288, 900 tokens 87.8 and 102; on the other side of
+    // the line Q4_K 4096 x 4096, 300 tokens 30.5 and 25.8; Q6_K 4096 x 12288, 512 tokens 75.7 and 55.3.  Long K is where the line is
+    // wrong: Q6_K 5120 x 25600, 512 tokens, 162 unsplit, 140 in three.
     if (a.m > 256 && 2 * tiles > a.sm_count) p.ksplit = 1;
     if (a.force_ksplit > 0 && a.force_ksplit <= p.nsb && plane_bytes * a.force_ksplit <= partial_space) p.ksplit = a.force_ksplit;
     const int pairs = a.sm_count / 2;

@@ -44,8 +44,11 @@ inline EncodeTiledFn encode_tiled_fn() {
     return fn;
 }
 
-// Waves x (K work per CTA + a fixed cost of about one and a half super-blocks for pipeline fill,
-// TMEM allocation and the epilogue), minimised over the split factor.
+// The GEMM's split factor: waves of tiles of 128 rows x (K work per CTA + a fixed cost of about one and a half super-blocks for
+// pipeline fill, TMEM allocation and the epilogue), minimised.  The kernel works on pairs of CTAs and cuts tokens finer than the
+// tiles counted here.  Against the best of eleven forced factors: within 1 % at six of nine shapes of 96..256 tokens (Q5_K 5120 x
+// 5120, 173 tokens: 24.1 us in three, 36.4 unsplit); behind it at Q4_K 24576 x 4096, 200 tokens (66.9 us, 57.6 unsplit), 12288 x 4096,
+// 128 tokens (33.2, 30.6 unsplit) and Q6_K 1024 x 4096, 256 tokens (21.5 in sixteen, 18.0 in four to eight).
 inline int choose_ksplit(int tiles, int nsb, int sm_count, size_t plane_bytes, size_t scratch_bytes, int max_tickets) {
     if (tiles > max_tickets) return 1;
     int best = 1;
@@ -64,9 +67,11 @@ inline int choose_ksplit(int tiles, int nsb, int sm_count, size_t plane_bytes, s
     return best;
 }
 
-// The decode kernel's split factor, fitted to measurements on B200 (times in units of one 128-row super-block,
-// ~1.45 us): a CTA costs its K share plus ~5 units of launch, pipeline fill and epilogue; every split adds a partial
-// tile the last CTA of the tile has to add, ~0.33 units per 16 tokens.  Ties go to the smaller factor.
+// The f16-tile decode kernel's split factor (qgemv_tc.cu; times in units of one 128-row super-block, ~1.45 us): a CTA costs its K
+// share plus ~5 units of launch, pipeline fill and epilogue; every split adds a partial tile the last CTA of the tile has to add,
+// ~0.33 units per 16 tokens.  Ties go to the smaller factor.  Q8_0, against the best forced factor: within 1 % from nine to 32 rows
+// (12288 x 4096, sixteen rows: 32.9 us unsplit, 39.6 in two; 4096 x 12288 31.4 in four, 37.2 in three); at 64 rows one split too many
+// (4096 x 4096 29.4 in four, 21.6 in three; 4096 x 12288 47.6 and 43.6).
 inline int choose_ksplit_decode(int tiles, int nsb, int sm_count, size_t plane_bytes, size_t scratch_bytes, int max_tickets,
                                 int tokens_per_tile) {
     if (tiles > max_tickets) return 1;
