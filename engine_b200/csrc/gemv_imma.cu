@@ -61,7 +61,7 @@ constexpr int kConsumerWarps = kGroups * kGroupWarps;
 constexpr int kConsumers = kConsumerWarps * 32;
 constexpr int kThreads = kConsumers + 32;      // + the producer warp
 constexpr int kTileRows = 16;                  // weight rows per tile (the M of m16n8k32)
-constexpr int kMaxStages = 8;                // of a CTA: one ring when it has one tile, else two (one per group) of half as many
+constexpr int kMaxStages = 8;                // of a CTA: in one ring, or in two (one per group) of half as many
 constexpr int kMaxSlots = 5;                   // tiles of a group whose partial sums may be waiting for their finisher
 constexpr int kMaxMembers = 8;                 // four column groups of two members
 constexpr int kSliceBytes = 768;               // image bytes per (member, super-block): 8 sub-blocks x 3 planes x 32
@@ -108,7 +108,7 @@ struct ImmaParams {
     int y_bf16;
     int accumulate;
     int k, n, nsb, members;
-    int stages, rings;          // stages per ring, and rings (1 when no CTA has a second tile)
+    int stages, rings;          // stages per ring, and rings: the consumer groups that take tiles
     int slots;                  // partial-sum slots per consumer group
     int tile_quotient, tile_remainder;   // tiles per CTA, and how many CTAs have one more
     int* status;
@@ -577,7 +577,7 @@ __host__ __device__ inline size_t imma_fixed_bytes(int members, int nsb, int slo
 
 // Where a CTA's stream of stages goes: chunk c (eight super-blocks) of its tiles, pairs of tiles interleaved chunk by chunk,
 // group g taking tile 2 i + g; an odd last tile is group 0's alone.  Each group has a ring of its own: a wait on one parity bit
-// is only safe for a warp that sees every phase of the barrier.
+// is only safe for a warp that sees every phase of the barrier.  With one ring group 0 takes every tile.
 struct Walk {
     int first, stage, phase;
     __device__ __forceinline__ int slot() const { return first + stage; }
@@ -685,8 +685,8 @@ __device__ __forceinline__ void gemv_imma_body(const CUtensorMap& wmap, const Im
             walk.step(stages);
         };
 #pragma unroll 1
-        for (int tile = 0; tile < tiles; tile += 2) {
-            const int both = tile + 1 < tiles ? 2 : 1;
+        for (int tile = 0; tile < tiles; tile += p.rings) {
+            const int both = min(p.rings, tiles - tile);
 #pragma unroll 1
             for (int step = 0; step < both * chunks; ++step) {
                 if (both == 1) {
@@ -785,7 +785,7 @@ __device__ __forceinline__ void gemv_imma_body(const CUtensorMap& wmap, const Im
         int slot = 0, slot_phase = 0, turn = 0;   // of the group's next tile: where its sums meet, and which warp finishes it
 
 #pragma unroll 1
-        for (int tile = group; tile < tiles; tile += kGroups) {
+        for (int tile = group; tile < tiles && group < p.rings; tile += p.rings) {
             const int row0 = (tile_begin + tile) * kTileRows;
             float acc[GROUPS][2], mins[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
@@ -952,8 +952,10 @@ struct Ring {
 };
 Ring ring_of(size_t stage_bytes, int members, int nsb, int tiles_per_cta, int wanted) {
     const int chunks = (nsb + kGroupWarps - 1) / kGroupWarps;
-    const int rings = tiles_per_cta > 1 ? 2 : 1, least = 2 / rings;
-    const int most = std::min(kMaxStages / rings, std::max(least, chunks * ((tiles_per_cta + 1) / 2)));   // no more than the CTA has use for
+    // A group with a single stage waits for every copy it asks for.  Where the images leave no more than that, one group has all the
+    // stages (4096 rows: Q4_K 4 x 12288 17.5 -> 13.5 us, 6 x 8192 14.7 -> 11.4; Q6_K 5 x 8192 18.1 -> 14.8).
+    const int rings = tiles_per_cta > 1 && imma_fixed_bytes(members, nsb, (2 + chunks) / chunks) + 4 * stage_bytes <= kSmemLimit ? 2 : 1, least = 2;
+    const int most = std::min(kMaxStages / rings, std::max(least, chunks * ((tiles_per_cta + rings - 1) / rings)));   // no more than the CTA has use for
     for (int stages = most; stages >= least; --stages) {
         if (wanted > 0 && stages * rings > wanted && stages > least) continue;
         // A warp that writes the slot of its group's tile T + slots has seen that tile's last stage, for which every warp of the group
