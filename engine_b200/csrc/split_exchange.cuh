@@ -52,14 +52,15 @@ __device__ __forceinline__ void exchange_reset(unsigned int* word, unsigned int*
     *word = 0u;
 }
 
-// Takes the lowest run of neighbouring shares off `mine`: items [first, last) of `items`.
+// Takes the lowest run of neighbouring shares off `mine`: items [first, last) of `items` (32-bit divisions, items * 24 below 2^31: the
+// 64-bit ones cost the batch kernel's Q6_K form, which has no register to spare, up to twenty bytes of spills).
 __device__ __forceinline__ void exchange_next(uint32_t& mine, int shares, int items, int& first, int& last) {
     const int begin = __ffs(static_cast<int>(mine)) - 1;
     const uint32_t rest = ~(mine >> begin);
     const int run = __ffs(static_cast<int>(rest)) - 1;   // at most 24 bits are set
     mine &= ~(((1u << run) - 1u) << begin);
-    first = static_cast<int>(static_cast<long long>(items) * begin / shares);
-    last = static_cast<int>(static_cast<long long>(items) * (begin + run) / shares);
+    first = static_cast<int>(static_cast<uint32_t>(items * begin) / static_cast<uint32_t>(shares));
+    last = static_cast<int>(static_cast<uint32_t>(items * (begin + run)) / static_cast<uint32_t>(shares));
 }
 
 }  // namespace ribn
