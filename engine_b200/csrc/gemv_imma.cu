@@ -686,7 +686,7 @@ __device__ __forceinline__ void gemv_imma_body(const CUtensorMap& wmap, const Im
         };
 #pragma unroll 1
         for (int tile = 0; tile < tiles; tile += p.rings) {
-            const int both = min(p.rings, tiles - tile);
+            const int both = p.rings == 2 && tile + 1 < tiles ? 2 : 1;
 #pragma unroll 1
             for (int step = 0; step < both * chunks; ++step) {
                 if (both == 1) {
@@ -785,7 +785,7 @@ __device__ __forceinline__ void gemv_imma_body(const CUtensorMap& wmap, const Im
         int slot = 0, slot_phase = 0, turn = 0;   // of the group's next tile: where its sums meet, and which warp finishes it
 
 #pragma unroll 1
-        for (int tile = group; tile < tiles && group < p.rings; tile += p.rings) {
+        for (int tile = group < p.rings ? group : tiles; tile < tiles; tile += p.rings) {
             const int row0 = (tile_begin + tile) * kTileRows;
             float acc[GROUPS][2], mins[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
