@@ -622,12 +622,15 @@ __device__ __forceinline__ bool store_unit(const GemmParams& p, int u, uint32_t 
             unsigned int* word = p.tickets + w.token_tile * 2 * p.row_pairs + w.row_tile;
             bars->word = word;
             // From the first to the last of the CTA's shares: one between them that another CTA adds gets the same bits from both, and
-            // one range costs the loops below (and the dequantisation beside them) no registers.
+            // one range costs the loops below (and the dequantisation beside them) no registers.  Cut before the wait: nearly always
+            // the CTA's own share.
+            const uint32_t shares = static_cast<uint32_t>(exchange_shares(ksplit)), items = static_cast<uint32_t>(tokens);
+            const uint32_t slice = static_cast<uint32_t>(w.k_slice);
+            bars->range = items * slice / shares | items * (slice + 1) / shares << 16;
             const uint32_t mine = exchange_arrive(word, ksplit, w.k_slice, p.patience_ns);
-            const int shares = exchange_shares(ksplit);
-            const int first = mine == 0 ? 0 : tokens * (__ffs(static_cast<int>(mine)) - 1) / shares;
-            const int last = mine == 0 ? 0 : tokens * (32 - __clz(static_cast<int>(mine))) / shares;
-            bars->range = static_cast<uint32_t>(first) | static_cast<uint32_t>(last) << 16;
+            if (mine == 0) bars->range = 0;
+            else if (mine != (slice < kExchangeShares ? 1u << slice : 0u))
+                bars->range = items * (__ffs(static_cast<int>(mine)) - 1) / shares | items * (32 - __clz(static_cast<int>(mine))) / shares << 16;
         }
         named_barrier_sync(2, kDequantWarps * 32);
         const int t_begin = static_cast<int>(bars->range & 0xffffu), t_end = static_cast<int>(bars->range >> 16);
