@@ -382,8 +382,8 @@ bool mma_serves(const ribn_ctx* ctx, const ribn_qweight* w, uint64_t k, uint64_t
 
 // Rows per launch of a call that the integer tensor-core kernel serves in smaller groups: long rows, of which eight images do not
 // fit shared memory, where only the integer-dot kernel is left.  That kernel rounds the rows to 15 bits instead of 22 and would give a
-// row other bits than a launch of fewer rows gives it.  It is also the slower one: Q8_0 4096 x 12288, eight rows, f32: 63.2 us, in
-// two launches of four 37.3; Q6_K 4096 x 11520 68.1 and 45.3, six rows 61.4 and 41.9.  0: not such a call (rows that are too long for
+// row other bits than a launch of fewer rows gives it.  It is also the slower one: Q8_0 4096 x 12288, eight rows, f32: 63.4 us, in
+// two launches of four 35.7; Q6_K 4096 x 11520 69.1 and 43.3, six rows 61.8 and 41.4.  0: not such a call (rows that are too long for
 // the integer-dot kernel as well stay with the f32 kernel, which beats groups of two: Q6_K 5120 x 25600, eight rows, 178 and 246 us).
 uint32_t imma_group(const ribn_ctx* ctx, const ribn_qweight* w, uint64_t k, uint64_t n, uint32_t members) {
     if (ctx->mma_gemv == 0 || ctx->gemv_path != 0 || ctx->imma_gemv == 0 || mma_serves(ctx, w, k, n, members)) return 0;
@@ -549,7 +549,10 @@ int enqueue_gemv(ribn_ctx* ctx, const ribn_qweight* w, uint64_t k, uint64_t n, c
     // activation pre-pass).  Its operands are f16: bf16 activations convert exactly and the weights'
     // rounding (2^-12) is below the one the caller applied to the activations (2^-9); f32 activations
     // would lose 13 bits, so they take it only on request.  Its scratch is the f16 copy of the activations.
-    // (Measured: a 16-token tile of the tensor-core kernel beats the integer-dot kernel's four rows from ~8 MB of weights up.)
+    // Rows too long for four of them in one narrow launch: four bf16 rows come here from tc_four_row_bytes of weights up (tcgen05 and the
+    // route below it: Q4_K 28672 values, 7.9 MB 24.6 and 22.2 us, 15.8 MB 26.3 and 27.8, 63 MB 51.5 and 68.6; Q8_0 17664, 9.2 MB 22.4 and
+    // 19.0, 18 MB 23.3 and 25.1, 73 MB 42.2 and 54.5; Q5_K 25600, 17 MB 26.3 and 26.4, 69 MB 50.4 and 64.8).  For Q6_K the line is
+    // wrong: 25600 values, 41 MB 71.7 and 40.4; 17664, 57 MB 96.3 and 54.3.
     if (tmem_serves(ctx, w, k, n, members, x_dtype))
         return enqueue_tmem(ctx, w, k, n, x, x_dtype, norm_weight != nullptr ? 1 : 0, norm_weight, eps, y, y_dtype, members, false);
     const bool mma = mma_serves(ctx, w, k, n, members);

@@ -111,11 +111,12 @@ void ribn_last_error_detail(const ribn_ctx *ctx, uint64_t *expected, uint64_t *a
  * (GemvMode, decode.rs:298-307).
  *   "gemv_path":    0 = choose per shape (default), 1 = f32 CUDA-core kernel only,
  *                   2 = integer-dot kernel only (error if the shape does not fit);
- *   "mma_gemv":     1 = calls of up to eight rows per launch (and wider f32 batches, in groups of eight) use the
- *                   mma.sync kernels where they serve the shape (Q4_K / Q5_K / Q6_K, 16-byte aligned rows, at least
- *                   16 output rows); 0 = leave them to the integer-dot kernel (default 1);
+ *   "mma_gemv":     1 = calls of up to eight rows per launch (and wider f32 batches, in groups of eight or of as many
+ *                   rows as fit a launch) use the mma.sync kernels where the weights start on a 16-byte boundary and
+ *                   have at least 16 output rows; 0 = leave them to the integer-dot kernel (default 1);
  *   "imma_gemv":    1 = those calls run on the integer instruction (quants as 8-bit operands, activations as
- *                   22-bit integers per 256-value slice); 0 = on the half2-unpack f16 kernel (default 1);
+ *                   22-bit integers per 256-value slice); 0 = Q4_K / Q5_K / Q6_K with rows of whole 16 bytes on the
+ *                   half2-unpack f16 kernel, the others on the integer-dot kernel (default 1);
  *                   "imma_max_members": largest such call (1..8, default 8);
  *   "mma_image_members": 3 = launches with more than 40 slices (rows x K / 256) or a gated input convert their
  *                   activations in a pre-pass launch, the others inside the GEMV kernel (default); another value =
@@ -259,8 +260,9 @@ int ribn_noalloc_status(int device, void *cuda_stream);
  *                                      silu(gate) * up (model_ops.rs:316-328)
  *   q and k (any two projections of one format) stored as one matrix: one launch, two outputs (split_rows)
  * All jobs share K; each is validated like ribn_gemv before anything is launched.  Served by the kernels ribn_gemv
- * uses (the integer tensor-core kernel for up to eight rows, the batch kernel from nine, the integer-dot kernel for
- * Q8_0); shapes that only the f32 kernel serves are refused with RIBN_E_INVALID_ARGUMENT (use the separate calls). */
+ * uses (the integer tensor-core kernel for up to eight rows, the batch kernels from nine, the integer-dot kernel for
+ * fewer than 16 output rows or weights off the 16-byte boundary); shapes that only the f32 kernel serves are refused
+ * with RIBN_E_INVALID_ARGUMENT (use the separate calls). */
 typedef struct ribn_gemv_job {
     uint32_t expected_type;      /* 0 = the weight's own type */
     const ribn_qweight* weight;
