@@ -15,7 +15,7 @@ e2e     = the same sweep through ribn_gemv_host_async + one ribn_synchronize per
           copies inside the timed region.
 cases   = every (format, shape, members) timed on its own (bursts over its cold ring), with the fraction of the
           measured HBM peak; `sustained` repeats the step for about a second so that the clock sampler sees it.
-parity  = largest error observed in this run, per kernel path, against the CPU checker (computed in the CPU-baseline leg).
+parity  = largest error observed in this run, per kernel path, against the CPU oracle (computed in the CPU-baseline leg).
 --impl reference = the CPU restatement of the reference's host path (dequantise a row, sequential
           f32 dot; oracle/ribn_oracle.c) on all host threads, on a bounded sample (a row range) of every GEMV of the sweep.
 """
@@ -587,7 +587,7 @@ def time_reference_cuda(cases, rings, acts, outs, capture, stream, step_bytes, r
 def cpu_baseline_leg(ctx=None):
     """Bounded CPU sample for the main arm: the M=1 GEMV of every (format, shape), reference host
     arithmetic, once single-threaded (the reference's host path is single-threaded) and once on all cores.
-    The CPU results double as the checker of this run's GPU results: `parity` holds the largest error observed
+    The CPU results double as the reference of this run's GPU results: `parity` holds the largest error observed
     per kernel path -- task metric |y - ref| / max(|ref|, sqrt(sum (w x)^2)) against the f64 product, the same
     against the reference's sequential f32 product, and the strict metric of oracle.max_rel_error_strict."""
     import oracle

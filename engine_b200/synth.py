@@ -10,7 +10,7 @@ Q8_0  (34 B):  d = f16(|N(0,1)| * 0.01); 32 int8 quants uniform in -128..127.
 
 A tensor is GGML dims [K, N]: N rows of K/block_elements consecutive blocks
 (crates/nvidia/src/quantized.rs:138-142).  The numpy generators are the ones parity tests use (the
-same bytes go to the CPU checker and to the GPU); the torch generator fills large random-init model
+same bytes go to the CPU oracle and to the GPU); the torch generator fills large random-init model
 weights directly in device memory.
 """
 from __future__ import annotations
