@@ -510,6 +510,19 @@ def test_long_rows_keep_their_bits_in_every_batch(ctx, gemv_path, vt, k):
         assert np.array_equal(y, one[:members]), members
 
 
+# images that leave one consumer group the whole ring, with three or four tiles per CTA and a ragged last one: the rows alone have two rings
+@pytest.mark.parametrize("vt,k,members", [(12, 12288, 4), (13, 12288, 4), (14, 8192, 6), (14, 256 * 45, 4), (8, 5888, 8), (8, 12288, 4), (8, 11232, 4)])
+def test_one_ring_with_several_tiles(ctx, gemv_path, vt, k, members):
+    if gemv_path != 0:
+        pytest.skip("the default path")
+    n = 148 * 16 * 3 + 197
+    weight = engine_b200.CudaQuantizedWeight(engine_b200.WeightTensorSpec.new("w", [k, n]), vt, synth.random_weight_device(vt, k, n, seed=k, device=ctx.device))
+    x = synth.random_activations(members, k, seed=k + 2)
+    one = np.concatenate([run_gemv(ctx, vt, weight, x[m:m + 1], n)[0] for m in range(members)])
+    y, _ = run_gemv(ctx, vt, weight, x, n)
+    assert np.isfinite(y).all() and np.array_equal(y, one)
+
+
 # projections of one gated or normalised input whose groups differ make their images anew
 @pytest.mark.parametrize("swiglu", [False, True])
 @pytest.mark.parametrize("members", [3, 7, 8])
